@@ -6,11 +6,10 @@
 // slot its pull reads before the step; the inlet face is pinned to the inlet equilibrium's mass and
 // momentum (:1313-1352); solid cells bounce back (:1602-1613).
 //
-// One thread per cell, 128 threads per CTA (a quarter of an 8^3 block), 4 CTAs per SM. A thread
-// pulls its 39 populations through the block's 27-entry neighbour table (|c| <= 3 < 8, so at most
-// one block hop) and parks them in shared memory while the 13-moment Newton solve (warm-started
-// from the cached multipliers) runs in registers; f_eq is parked beside them for the rarely taken
-// post-collision paths. Then WALE from the 6 face neighbours' previous velocity, the Mach-pocket
+// One thread per cell, 128 threads per CTA (a quarter of an 8^3 block). A thread pulls its 39
+// populations through the block's 27-entry neighbour table (|c| <= 3 < 8, so at most one block hop)
+// and parks them in shared memory while the 13-moment Newton solve (warm-started from the cached
+// multipliers) runs in registers. Then WALE from the 6 face neighbours' previous velocity, the Mach-pocket
 // viscosity, positivity clamp and realizability guard, the mirror split, the entropic alpha, the
 // KBC update and the post-collision guards. It writes 39 populations, rho, u and the 13
 // multipliers. The step is bound by FP32 issue (a Newton sweep is 117 exponentials, an entropy
@@ -257,30 +256,250 @@ __device__ __forceinline__ float fi_row(float rho, const float (&la)[13], const 
   return maxc(rho * row[3].x * kexp<FAST>(jclamp(lda_row<FAST>(la, row), -20.0f, 20.0f)), 1e-15f);
 }
 
-// The fast path's full Newton pass: at the multipliers la, the moments d = sum_k f_k b_k and the
-// Hessian of the dual problem H = sum_k f_k b_k b_k^T (b_k = (1, basis row k)), H packed lower
-// triangular, (i, j <= i) at i (i + 1) / 2 + j.
-__device__ __forceinline__ void newton_pass(const Tables& T, float rho, const float (&la)[13], float (&d)[13],
-                                            float (&H)[91]) {
-#pragma unroll
-  for (int m = 0; m < 13; ++m) d[m] = 0.0f;
-#pragma unroll
-  for (int n = 0; n < 91; ++n) H[n] = 0.0f;
-#pragma unroll 1
-  for (int k = 0; k < Q; ++k) {
-    const float4* row = T.b[k];
-    const float fi = fi_row<true>(rho, la, row);
-    const float4 r0 = row[0], r1 = row[1], r2 = row[2];
-    const float b[13] = {1.0f, r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w, r2.x, r2.y, r2.z, r2.w};
-#pragma unroll
-    for (int i = 0; i < 13; ++i) {
-      const float fb = fi * b[i];
-      d[i] += fb;
-#pragma unroll
-      for (int j = 0; j <= i; ++j) H[i * (i + 1) / 2 + j] = __fmaf_rn(fb, b[j], H[i * (i + 1) / 2 + j]);
-    }
-  }
+// ---- the fast path's Newton pass in raw moments of the direction pairs ------------------------
+// A full Newton step needs f_k = rho w_k exp(lda_k) of the 39 directions, their 13 moments and the
+// Hessian of the dual problem, H = sum_k f_k b_k b_k^T. Run over a basis table (one exponential, 12
+// multiply-adds and 104 accumulations per direction) that is ~5,200 instructions. Here the sums use
+// what the lattice is: in the unshifted basis (1, c, c_a^2, c_a c_b, |c|^2 c_a) every entry of H is
+// a raw moment, a raw moment needs only the even part f_k + f_opp or the odd part f_k - f_opp of a
+// pair, all but a few of the 19 pairs contribute with integer factors or not at all, and the 91
+// entries are 44 different moments. lda_k = E +- O splits the same way. Everything is unrolled over
+// the pairs (compile-time velocities), ~600 instructions per pass, the populations in registers.
+// Newton steps do not depend on the basis; multipliers, targets and the residual test stay in the
+// shifted basis of the reference (la[0..12]).
+// Measured: see k_kbc_step.
+
+// first direction (positive leading component) of each pair, in the order the moments below use
+__host__ __device__ constexpr int kpos(int p) {
+  constexpr int t[19] = {2, 4, 6, 14, 13, 12, 11, 16, 18, 20, 24, 23, 28, 27, 32, 31, 34, 36, 38};
+  return t[p];
 }
+constexpr bool kpos_ok() {
+  for (int p = 0; p < 19; ++p) {
+    const int k = kpos(p);
+    const int lead = kcx(k) != 0 ? kcx(k) : kcy(k) != 0 ? kcy(k) : kcz(k);
+    if (lead <= 0 || kopp(kopp(k)) != k) return false;
+    for (int q = 0; q < p; ++q)
+      if (kpos(q) == k || kopp(kpos(q)) == k) return false;
+  }
+  return true;
+}
+static_assert(kpos_ok(), "pair order");
+__host__ __device__ constexpr int kc2(int k) { return kcx(k) * kcx(k) + kcy(k) * kcy(k) + kcz(k) * kcz(k); }
+__host__ __device__ constexpr int kfam(int k) {  // the five shells |c|^2 = 1, 3, 4, 8, 9
+  return kc2(k) == 1 ? 0 : kc2(k) == 3 ? 1 : kc2(k) == 4 ? 2 : kc2(k) == 8 ? 3 : 4;
+}
+
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// f_k = rho w_k exp(lda_k) at the multipliers la; false when some |lda_k| may exceed 20, where the
+// reference clamps it (the caller then takes the table path, which clamps)
+__device__ __forceinline__ bool eq_pops(float rho, const float (&la)[13], float (&f)[Q]) {
+  constexpr float L2E = 1.44269504088896341f, TEN3 = 5.0f * CS2;
+  // unshifted multipliers, in units of log 2
+  const float l0 = L2E * __fmaf_rn(-CS2, (la[4] + la[5]) + la[6], la[0]);
+  float g1[3], q[3], m2[3], mx[3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    g1[a] = L2E * __fmaf_rn(-TEN3, la[10 + a], la[1 + a]);
+    q[a] = L2E * la[10 + a];
+    m2[a] = L2E * la[4 + a];
+    mx[a] = L2E * la[7 + a];
+  }
+  // |lda| <= |l0| + 9 |m2| + 4 |mx| + 3 |g1| + 27 |q| over the directions
+  const float bound = fabsf(l0) + 9.0f * (fabsf(m2[0]) + fabsf(m2[1]) + fabsf(m2[2])) +
+                      4.0f * (fabsf(mx[0]) + fabsf(mx[1]) + fabsf(mx[2])) +
+                      3.0f * (fabsf(g1[0]) + fabsf(g1[1]) + fabsf(g1[2])) +
+                      27.0f * (fabsf(q[0]) + fabsf(q[1]) + fabsf(q[2]));
+  if (!(bound <= 20.0f * L2E)) return false;
+  float g[5][3];
+  constexpr float c2f[5] = {1.0f, 3.0f, 4.0f, 8.0f, 9.0f};
+#pragma unroll
+  for (int s = 0; s < 5; ++s)
+#pragma unroll
+    for (int a = 0; a < 3; ++a) g[s][a] = __fmaf_rn(c2f[s], q[a], g1[a]);
+  f[0] = rho * kw(0) * ex2(l0);
+#pragma unroll
+  for (int p = 0; p < 19; ++p) {
+    const int k = kpos(p), kb = kopp(k), s = kfam(k);
+    const int c[3] = {kcx(k), kcy(k), kcz(k)};
+    float E = l0;
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+      if (c[a] != 0) E = __fmaf_rn(float(c[a] * c[a]), m2[a], E);
+    if (c[0] * c[1] != 0) E = __fmaf_rn(float(c[0] * c[1]), mx[0], E);
+    if (c[0] * c[2] != 0) E = __fmaf_rn(float(c[0] * c[2]), mx[1], E);
+    if (c[1] * c[2] != 0) E = __fmaf_rn(float(c[1] * c[2]), mx[2], E);
+    float O = 0.0f;
+    bool first = true;
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+      if (c[a] != 0) {
+        O = first ? float(c[a]) * g[s][a] : __fmaf_rn(float(c[a]), g[s][a], O);
+        first = false;
+      }
+    const float rw = rho * kw(k);
+    f[k] = rw * ex2(E + O);
+    f[kb] = rw * ex2(E - O);
+  }
+  return true;
+}
+
+// the even and odd pair sums by shell: 1 = (1,0,0), T = (1,1,1), 2 = (2,0,0), D = (2,2,0), 3 = (3,0,0)
+struct PairSums {
+  float n0;
+  float e1[3], t[4], e2[3], d[3][2], e3[3];  // f_k + f_opp; d: planes xy, xz, yz, signs (+,+) and (+,-)
+  float o1[3], u[4], o2[3], w[3][2], o3[3];  // f_k - f_opp
+};
+__device__ __forceinline__ void pair_sums(const float (&f)[Q], PairSums& S) {
+  S.n0 = f[0];
+  auto pr = [&](int p, float& e, float& o) {
+    const int k = kpos(p), kb = kopp(k);
+    e = f[k] + f[kb];
+    o = f[k] - f[kb];
+  };
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    pr(a, S.e1[a], S.o1[a]);
+    pr(7 + a, S.e2[a], S.o2[a]);
+    pr(16 + a, S.e3[a], S.o3[a]);
+    pr(10 + 2 * a, S.d[a][0], S.w[a][0]);
+    pr(11 + 2 * a, S.d[a][1], S.w[a][1]);
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) pr(3 + i, S.t[i], S.u[i]);
+}
+
+// One Newton pass at populations f: the residual r of the raw moments (targets: rho, u with
+// P_ab = rho (u_a u_b + cs2 delta), Q_a = rho u_a (u^2 + 5 cs2)); returns its square norm in the
+// reference's shifted basis. hess(): the raw-moment Hessian, packed as newton_solve takes it.
+struct NewtonPass {
+  PairSums S;
+  float T, XY[3], DXY[3], Bx[3], Qt[3], A[3], Axyz, W[3][2];
+  float M2[3], Mx[3];
+  __device__ __forceinline__ float residual(const float (&f)[Q], float rho, float ux, float uy, float uz, float (&r)[13]) {
+    pair_sums(f, S);
+    T = (S.t[0] + S.t[1]) + (S.t[2] + S.t[3]);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      XY[i] = S.d[i][0] + S.d[i][1];
+      DXY[i] = S.d[i][0] - S.d[i][1];
+      W[i][0] = S.w[i][0] + S.w[i][1];  // odd (2,2,0) sums: first axis of the plane,
+      W[i][1] = S.w[i][0] - S.w[i][1];  // second axis
+    }
+    // planes xy, xz, yz: axis a lies in two of them
+    Bx[0] = XY[0] + XY[1]; Bx[1] = XY[0] + XY[2]; Bx[2] = XY[1] + XY[2];
+    const float t01 = S.t[0] + S.t[1], t23 = S.t[2] + S.t[3], t02 = S.t[0] + S.t[2], t13 = S.t[1] + S.t[3];
+    Qt[0] = t01 - t23;                                // xy signs + + - -
+    Qt[1] = t02 - t13;                                // xz       + - + -
+    Qt[2] = (S.t[0] + S.t[3]) - (S.t[1] + S.t[2]);    // yz       + - - +
+    A[0] = (S.u[0] + S.u[1]) + (S.u[2] + S.u[3]);
+    A[1] = (S.u[0] + S.u[1]) - (S.u[2] + S.u[3]);
+    A[2] = (S.u[0] + S.u[2]) - (S.u[1] + S.u[3]);
+    Axyz = (S.u[0] + S.u[3]) - (S.u[1] + S.u[2]);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) M2[a] = __fmaf_rn(9.0f, S.e3[a], __fmaf_rn(4.0f, S.e2[a] + Bx[a], S.e1[a] + T));
+#pragma unroll
+    for (int i = 0; i < 3; ++i) Mx[i] = __fmaf_rn(4.0f, DXY[i], Qt[i]);
+    const float M0 = ((S.n0 + T) + ((S.e1[0] + S.e1[1]) + S.e1[2])) + (((S.e2[0] + S.e2[1]) + S.e2[2]) +
+                     ((XY[0] + XY[1]) + XY[2])) + ((S.e3[0] + S.e3[1]) + S.e3[2]);
+    const float V[3] = {W[0][0] + W[1][0], W[0][1] + W[2][0], W[1][1] + W[2][1]};  // odd (2,2,0) sums with c_a
+    float j[3], qm[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      j[a] = __fmaf_rn(3.0f, S.o3[a], __fmaf_rn(2.0f, S.o2[a] + V[a], S.o1[a] + A[a]));
+      qm[a] = __fmaf_rn(27.0f, S.o3[a], __fmaf_rn(16.0f, V[a], __fmaf_rn(8.0f, S.o2[a], __fmaf_rn(3.0f, A[a], S.o1[a]))));
+    }
+    const float u[3] = {ux, uy, uz};
+    const float usq = ux * ux + uy * uy + uz * uz;
+    r[0] = rho - M0;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      r[1 + a] = rho * u[a] - j[a];
+      r[4 + a] = rho * __fmaf_rn(u[a], u[a], CS2) - M2[a];
+      r[10 + a] = rho * u[a] * (usq + 5.0f * CS2) - qm[a];
+    }
+    r[7] = rho * ux * uy - Mx[0];
+    r[8] = rho * ux * uz - Mx[1];
+    r[9] = rho * uy * uz - Mx[2];
+    m0 = M0; jm[0] = j[0]; jm[1] = j[1]; jm[2] = j[2]; qmom[0] = qm[0]; qmom[1] = qm[1]; qmom[2] = qm[2];
+    float res = r[0] * r[0];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const float s2 = __fmaf_rn(-CS2, r[0], r[4 + a]), sq = __fmaf_rn(-5.0f * CS2, r[1 + a], r[10 + a]);
+      res = __fmaf_rn(r[1 + a], r[1 + a], res);
+      res = __fmaf_rn(s2, s2, res);
+      res = __fmaf_rn(r[7 + a], r[7 + a], res);
+      res = __fmaf_rn(sq, sq, res);
+    }
+    return res;
+  }
+  float m0, jm[3], qmom[3];
+  // unknowns: 0: 1; 1-3: c; 4-6: c_a^2; 7-9: c_x c_y, c_x c_z, c_y c_z; 10-12: |c|^2 c
+  __device__ __forceinline__ void hess(float (&H)[91]) const {
+    auto at = [&](int i, int j2) -> float& { return i >= j2 ? H[i * (i + 1) / 2 + j2] : H[j2 * (j2 + 1) / 2 + i]; };
+    // plane index of axes (a, b) and the cross moments' positions
+    constexpr int pl[3][3] = {{-1, 0, 1}, {0, -1, 2}, {1, 2, -1}};
+    at(0, 0) = m0;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      at(1 + a, 0) = jm[a];
+      at(4 + a, 0) = M2[a];
+      at(7 + a, 0) = Mx[a];
+      at(10 + a, 0) = qmom[a];
+    }
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      // c_a c_a, c_a^2 c_a^2, |c|^2 c_a c_a, |c|^4 c_a c_a
+      at(1 + a, 1 + a) = M2[a];
+      at(4 + a, 4 + a) = __fmaf_rn(81.0f, S.e3[a], __fmaf_rn(16.0f, S.e2[a] + Bx[a], S.e1[a] + T));
+      at(10 + a, 1 + a) = __fmaf_rn(81.0f, S.e3[a], __fmaf_rn(32.0f, Bx[a], __fmaf_rn(16.0f, S.e2[a], __fmaf_rn(3.0f, T, S.e1[a]))));
+      at(10 + a, 10 + a) = __fmaf_rn(729.0f, S.e3[a], __fmaf_rn(256.0f, Bx[a], __fmaf_rn(64.0f, S.e2[a], __fmaf_rn(9.0f, T, S.e1[a]))));
+      // odd: c_a^2 c_a and c_a^2 |c|^2 c_a
+      const float V = a == 0 ? W[0][0] + W[1][0] : a == 1 ? W[0][1] + W[2][0] : W[1][1] + W[2][1];
+      at(4 + a, 1 + a) = __fmaf_rn(27.0f, S.o3[a], __fmaf_rn(8.0f, S.o2[a] + V, S.o1[a] + A[a]));
+      at(10 + a, 4 + a) = __fmaf_rn(243.0f, S.o3[a], __fmaf_rn(64.0f, V, __fmaf_rn(32.0f, S.o2[a], __fmaf_rn(3.0f, A[a], S.o1[a]))));
+    }
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+      for (int b = 0; b < 3; ++b) {
+        if (a == b) continue;
+        const int p = pl[a][b];
+        if (b < a) {
+          at(1 + a, 1 + b) = Mx[p];
+          at(4 + a, 4 + b) = __fmaf_rn(16.0f, XY[p], T);                       // c_a^2 c_b^2
+          at(10 + a, 10 + b) = __fmaf_rn(256.0f, DXY[p], 9.0f * Qt[p]);        // |c|^4 c_a c_b
+          at(7 + p, 7 + p) = at(4 + a, 4 + b);
+        }
+        at(10 + a, 1 + b) = __fmaf_rn(32.0f, DXY[p], 3.0f * Qt[p]);            // |c|^2 c_a c_b
+        // (2,2,0) odd sum of plane p with c_a: first axis W[p][0], second W[p][1]
+        const float wa = a < b ? W[p][0] : W[p][1];
+        const float aab = __fmaf_rn(8.0f, wa, A[a]), aabq = __fmaf_rn(64.0f, wa, 3.0f * A[a]);
+        at(4 + b, 1 + a) = aab;                                                // c_b^2 c_a
+        at(10 + a, 4 + b) = aabq;                                              // c_b^2 |c|^2 c_a
+        // c_a c_b times c_b gives c_b^2 c_a
+        at(7 + p, 1 + b) = aab;
+        at(10 + b, 7 + p) = aabq;
+        at(7 + p, 4 + a) = __fmaf_rn(16.0f, DXY[p], Qt[p]);                    // c_a^3 c_b
+      }
+    // entries with all three axes: only the (1,1,1) shell
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const int p = a == 0 ? 2 : a == 1 ? 1 : 0;  // the plane without axis a
+      at(7 + p, 1 + a) = Axyz;
+      at(10 + a, 7 + p) = 3.0f * Axyz;
+      at(7 + p, 4 + a) = Qt[p];                   // c_a^2 c_b c_c
+    }
+    at(8, 7) = Qt[2];  // c_x^2 c_y c_z
+    at(9, 7) = Qt[1];  // c_x c_y^2 c_z
+    at(9, 8) = Qt[0];  // c_x c_y c_z^2
+  }
+};
 
 // Solves H x = r in place (r becomes x) by a Cholesky factorisation of the packed H; false when
 // H is not numerically positive definite.
@@ -324,7 +543,7 @@ __device__ __forceinline__ bool newton_solve(float (&H)[91], float (&r)[13]) {
 // start), keeping the sweeps as its fallback.
 template <bool FAST = false>
 __device__ __forceinline__ void solve_lambdas(const Tables& T, float rho, float ux, float uy, float uz, float (&la)[13],
-                                              float warm_gate = 100.0f) {
+                                              float (&fe)[FAST ? Q : 1], float warm_gate = 100.0f) {
   const float OMEGA = 1.5f, F_FLOOR_EQ = 1e-15f;
   const float eps = 1.1920928955078125e-7f;
   const float TOL_SQ = 507.0f * eps * eps * rho * rho * (FAST ? KBC_FAST_TOL_SCALE : 1.0f);
@@ -348,14 +567,10 @@ __device__ __forceinline__ void solve_lambdas(const Tables& T, float rho, float 
     bool cold = la[0] != la[0];
     if (cold) poly_start();
     for (int it = 0; it < KBC_NEWTON_MAX; ++it) {
-      float d[13], H[91], r[13];
-      newton_pass(T, rho, la, d, H);
-      float res = 0.0f;
-#pragma unroll
-      for (int m = 0; m < 13; ++m) {
-        r[m] = mt[m] - d[m];
-        res = __fmaf_rn(r[m], r[m], res);
-      }
+      if (!eq_pops(rho, la, fe)) break;
+      NewtonPass np;
+      float r[13];
+      const float res = np.residual(fe, rho, ux, uy, uz, r);
       if (res < TOL_SQ) return;
       if (!cold && it == 0 && res > warm_gate * TOL_SQ) {
         // staleness gate on the warm start (physics_utils.jl:603-634)
@@ -363,7 +578,13 @@ __device__ __forceinline__ void solve_lambdas(const Tables& T, float rho, float 
         cold = true;
         continue;
       }
+      float H[91];
+      np.hess(H);
       if (!newton_solve(H, r)) break;
+      // back to the shifted basis of la
+      r[0] = __fmaf_rn(CS2, (r[4] + r[5]) + r[6], r[0]);
+#pragma unroll
+      for (int a = 0; a < 3; ++a) r[1 + a] = __fmaf_rn(5.0f * CS2, r[10 + a], r[1 + a]);
 #pragma unroll
       for (int m = 0; m < 13; ++m) la[m] += jclamp(r[m], -2.0f, 2.0f);
     }
@@ -437,6 +658,10 @@ __device__ __forceinline__ void solve_lambdas(const Tables& T, float rho, float 
 #pragma unroll
     for (int m = 0; m < 13; ++m) res += (mt[m] - d[m]) * (mt[m] - d[m]);
     if (res < TOL_SQ) break;
+  }
+  if constexpr (FAST) {
+#pragma unroll
+    for (int k = 0; k < Q; ++k) fe[k] = fi_row<FAST>(rho, la, T.b[k]);
   }
 }
 
@@ -587,6 +812,178 @@ __device__ __forceinline__ bool alpha_taylor(const Tables& T, const float* sf, c
   return true;
 }
 
+// ---- alpha of the fast path from a series of the entropy ---------------------------------------
+// The bisection needs the sign of H(alpha) - H_pre, H = sum_k f_k ln(f_k / w_k), at 12 values of
+// alpha. Near equilibrium that difference is ~1e-8 while the sums carry ~1e-7 of FP32 rounding, and
+// each evaluation is 39 logarithms. With f_k = fe_k (1 + y_k) and ln(fe_k / w_k) = ln(rho corr) +
+// lda_k, H splits into the multipliers times the moments of f - fe and sum fe g(y), g(y) = (1 + y)
+// ln(1 + y) - y = y^2/2 - y^3/6 + y^4/12 - ...; f - fe = coeff_s s + coeff_h h with s even and h odd in
+// the pair, so sum fe g(y) is a polynomial in coeff_h whose coefficients are 12 sums over the pairs,
+// gathered once. Mass and momentum of s and h are zero (f_eq has the cell's), which leaves the stress
+// moments of s and the energy-flux moments of h. The differences then come out of small quantities
+// alone, and the 12 evaluations are a quartic each. The first dropped term is fe y^5 / 20: at
+// |y| <= kSeriesRoot, which only the light shells reach (w <= 1/432), that is below 4e-8, a tenth of
+// the rounding of the sums it replaces. So the series decides where |y| stays below kSeriesRoot for
+// |coeff_h| <= kRootReach and the root lies there, and below kSeriesFar over the whole bracket
+// (|coeff_h| <= 7), whose far end only has to have the right sign; elsewhere the sums of logarithms
+// decide.
+constexpr float kSeriesRoot = 0.2f, kSeriesFar = 0.7f, kRootReach = 2.5f;
+struct AlphaSeries {
+  float a20 = 0.0f, a11 = 0.0f, a02 = 0.0f, a30 = 0.0f, a21 = 0.0f, a12 = 0.0f, a03 = 0.0f;
+  float a40 = 0.0f, a31 = 0.0f, a22 = 0.0f, a13 = 0.0f, a04 = 0.0f;
+  float P[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f}, qf[3] = {0.0f, 0.0f, 0.0f};
+  float h_sq = 0.0f, y_root = 0.0f, y_far = 0.0f;  // the largest |y| bounds
+  static __device__ __forceinline__ float rcp(float v) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+    return r;
+  }
+  // the |y| bounds of the cell; true where they admit the series
+  __device__ __forceinline__ bool admits(const float* sf, const float (&fe)[Q]) {
+    y_root = y_far = fabsf(sf[0] - fe[0]) * rcp(fe[0]);
+#pragma unroll
+    for (int p = 0; p < 19; ++p) {
+      const int k = kpos(p), kb = kopp(k);
+      const float df = sf[k * kThreads] - fe[k], db = sf[kb * kThreads] - fe[kb];
+      const float s = 0.5f * fabsf(df + db), h = 0.5f * fabsf(df - db), r = rcp(fminf(fe[k], fe[kb]));
+      y_root = fmaxf(y_root, __fmaf_rn(kRootReach, h, s) * r);
+      y_far = fmaxf(y_far, __fmaf_rn(7.0f, h, s) * r);
+    }
+    return y_root <= kSeriesRoot && y_far <= kSeriesFar;
+  }
+  __device__ __forceinline__ void gather(const float* sf, const float (&fe)[Q]) {
+    {
+      const float s = sf[0] - fe[0], y = s * rcp(fe[0]), s2 = s * y;
+      a20 = s2;
+      a30 = s2 * y;
+      a40 = s2 * y * y;
+    }
+#pragma unroll
+    for (int p = 0; p < 19; ++p) {
+      const int k = kpos(p), kb = kopp(k);
+      const float df = sf[k * kThreads] - fe[k], db = sf[kb * kThreads] - fe[kb];
+      const float s = 0.5f * (df + db), h = 0.5f * (df - db);
+      const float rp = rcp(fe[k]), rm = rcp(fe[kb]);
+      const float s2 = s * s, sh = s * h, h2 = h * h;
+      const float R1 = rp + rm, Q1 = rp - rm;
+      a20 = __fmaf_rn(s2, R1, a20);
+      a11 = __fmaf_rn(sh, Q1, a11);
+      a02 = __fmaf_rn(h2, R1, a02);
+      const float rp2 = rp * rp, rm2 = rm * rm;
+      const float sR2 = s * (rp2 + rm2), hQ2 = h * (rp2 - rm2);
+      a30 = __fmaf_rn(s2, sR2, a30);
+      a21 = __fmaf_rn(s2, hQ2, a21);
+      a12 = __fmaf_rn(h2, sR2, a12);
+      a03 = __fmaf_rn(h2, hQ2, a03);
+      const float rp3 = rp2 * rp, rm3 = rm2 * rm;
+      const float s2R3 = s2 * (rp3 + rm3), h2R3 = h2 * (rp3 + rm3), shQ3 = sh * (rp3 - rm3);
+      a40 = __fmaf_rn(s2, s2R3, a40);
+      a31 = __fmaf_rn(s2, shQ3, a31);
+      a22 = __fmaf_rn(h2, s2R3, a22);
+      a13 = __fmaf_rn(h2, shQ3, a13);
+      a04 = __fmaf_rn(h2, h2R3, a04);
+      const int c[3] = {kcx(k), kcy(k), kcz(k)};
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        if (c[a] != 0) P[a] = __fmaf_rn(2.0f * float(c[a] * c[a]), s, P[a]);
+        if (c[a] != 0) qf[a] = __fmaf_rn(2.0f * float(kc2(k) * c[a]), h, qf[a]);
+      }
+      if (c[0] * c[1] != 0) P[3] = __fmaf_rn(2.0f * float(c[0] * c[1]), s, P[3]);
+      if (c[0] * c[2] != 0) P[4] = __fmaf_rn(2.0f * float(c[0] * c[2]), s, P[4]);
+      if (c[1] * c[2] != 0) P[5] = __fmaf_rn(2.0f * float(c[1] * c[2]), s, P[5]);
+      h_sq = __fmaf_rn(2.0f, h2, h_sq);
+    }
+  }
+  // kernel_entropic_d3q39.jl:417-442 and the clamp of :3144-3150 on the gathered series; false where
+  // the root lies beyond its reach
+  __device__ __forceinline__ bool solve(const float (&la)[13], float beta, float& alpha) const {
+    alpha = 2.0f;
+    if (!(h_sq > 1e-20f)) return true;
+    const float cs = 1.0f - 2.0f * beta, cs2 = cs * cs, cs3 = cs2 * cs;
+    float ls = 0.0f, lq = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 6; ++i) ls = __fmaf_rn(la[4 + i], P[i], ls);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) lq = __fmaf_rn(la[10 + a], qf[a], lq);
+    // G(c) = H - H_pre at coeff_h = c, the arriving populations being coeff_s = coeff_h = 1
+    const float pre = ((0.5f * a20 + a11) + 0.5f * a02) -
+                      ((a30 * (1.0f / 6.0f) + 0.5f * a21) + (0.5f * a12 + a03 * (1.0f / 6.0f))) +
+                      ((a40 * (1.0f / 12.0f) + a31 * (1.0f / 3.0f)) + (0.5f * a22 + a13 * (1.0f / 3.0f)) + a04 * (1.0f / 12.0f));
+    const float c1 = cs * a11 - 0.5f * cs2 * a21 + cs3 * (1.0f / 3.0f) * a31 + lq;
+    const float c2 = 0.5f * ((a02 - cs * a12) + cs2 * a22);
+    const float c3 = cs * (1.0f / 3.0f) * a13 - (1.0f / 6.0f) * a03;
+    const float c4 = (1.0f / 12.0f) * a04;
+    const float c0 = (0.5f * cs2 * a20 - cs3 * (1.0f / 6.0f) * a30 + cs2 * cs2 * (1.0f / 12.0f) * a40) - pre +
+                     ((cs - 1.0f) * ls - lq);
+    auto G = [&](float al) {
+      const float c = 1.0f - 2.0f * beta * al;
+      return __fmaf_rn(c, __fmaf_rn(c, __fmaf_rn(c, __fmaf_rn(c, c4, c3), c2), c1), c0);
+    };
+    const float inv_2beta = 0.5f / fmaxf(beta, 0.01f);
+    float lo = fmaxf(inv_2beta - 0.1f, 0.1f), hi = fmaxf(inv_2beta + 3.0f, 4.0f);
+    const float G_lo = G(lo), G_hi = G(hi);
+    alpha = inv_2beta;
+    bool decided = y_far <= kSeriesRoot;
+    if ((G_lo < 0.0f && G_hi > 0.0f) || (G_lo > 0.0f && G_hi < 0.0f)) {
+      const bool neg = G_lo < 0.0f;
+#pragma unroll 1
+      for (int it = 0; it < 10; ++it) {
+        const float al = 0.5f * (lo + hi), g = G(al);
+        if (neg ? g < 0.0f : g > 0.0f) lo = al;
+        else hi = al;
+        if ((hi - lo) < 0.005f * (inv_2beta + 1e-6f)) break;
+      }
+      alpha = 0.5f * (lo + hi);
+      decided = decided || fabsf(1.0f - 2.0f * beta * alpha) <= kRootReach;
+    }
+    if (!(alpha > 0.0f)) alpha = inv_2beta;
+    alpha = jclamp(alpha, inv_2beta, 6.0f);
+    return decided;
+  }
+};
+
+// The bisection by sums of logarithms with the cell's a_k and h_p in registers (the fast path where
+// the series does not decide): the evaluations of alpha_bisection unrolled, ~200 instructions each
+// instead of ~550 over the shared columns, in units of log 2 (only signs of differences matter).
+__device__ __forceinline__ float lg2(float v) {
+  float r;
+  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+  return r;
+}
+__device__ __forceinline__ float entropy_term(float f, int k, float H) {
+  const float fk = fmaxf(f, F_FLOOR);
+  return __fmaf_rn(fk, lg2(fk * (1.0f / kw(k))), H);
+}
+__device__ __forceinline__ float entropy_regs(const float (&av)[Q], const float (&hv)[19], float c) {
+  float H0 = entropy_term(av[0], 0, 0.0f), H1 = 0.0f;
+#pragma unroll
+  for (int p = 0; p < 19; ++p) {
+    const int k = kpos(p), kb = kopp(k);
+    H0 = entropy_term(__fmaf_rn(c, hv[p], av[k]), k, H0);
+    H1 = entropy_term(__fmaf_rn(-c, hv[p], av[kb]), kb, H1);
+  }
+  return H0 + H1;
+}
+__device__ __forceinline__ float alpha_bisection_regs(const float (&av)[Q], const float (&hv)[19], float beta, float H_pre) {
+  const float inv_2beta = 0.5f / fmaxf(beta, 0.01f);
+  float lo = fmaxf(inv_2beta - 0.1f, 0.1f), hi = fmaxf(inv_2beta + 3.0f, 4.0f);
+  float d_lo = 0.0f;
+#pragma unroll 1
+  for (int it = -2; it < 10; ++it) {
+    const float al = it == -2 ? lo : it == -1 ? hi : 0.5f * (lo + hi);
+    const float d = entropy_regs(av, hv, 1.0f - 2.0f * beta * al) - H_pre;
+    if (it == -2) { d_lo = d; continue; }
+    if (it == -1) {
+      if (!(d_lo * d < 0.0f)) return inv_2beta;
+      continue;
+    }
+    if (d * d_lo > 0.0f) lo = al;
+    else hi = al;
+    if ((hi - lo) < 0.005f * (inv_2beta + 1e-6f)) break;
+  }
+  return 0.5f * (lo + hi);
+}
+
 // The face fill (kernel_entropic_d3q39.jl:983-1278 at the default boundary options): one thread per
 // pull whose source lies outside the domain; its value goes to the ghost slot the pull reads (the
 // slot (source cell, k) has exactly one reader, the source + c_k).
@@ -680,6 +1077,16 @@ __device__ __forceinline__ void svv_axis(const SvvView a, const Tables& T, const
   }
 }
 
+// What bounds the fast instances: FP32 issue. They run ~5,500 thread-instructions per cell (two to
+// three Newton passes of ~600 and one or two Cholesky solves of ~650, alpha ~1,200, the rest pull,
+// WALE and update) at 168 registers, three CTAs per SM, issue 51 % active (no_instruction and wait
+// stalls: the body is straight-line code). The body is unrolled over the pairs with the 39
+// equilibrium values in registers; the rare paths (guards, clamps, HRR, the other alpha solvers)
+// read the shared columns. Measured on a 96^3 periodic box, two steps per call: 2,660 us with the
+// Newton pass over the basis table, alpha from sums of logarithms over the columns and a trip to
+// memory per pulled direction; 451 us now while alpha comes from the series, 1,040 us (3,370 before)
+// on a developed flow whose deviations are of the order of f_eq, so that every alpha comes from the
+// logarithms. Distance from the 64-bit step after two steps: velocity 3.1e-5 against 2.9e-3 before.
 // SVV: the spectral vanishing viscosity is compiled in (a.svv_x or a.svv_yz > 0).
 template <bool EDGES, bool FAST, bool SVV = false>
 __global__ void __launch_bounds__(kThreads, FAST ? KBC_FAST_MIN_BLOCKS : KBC_MIN_BLOCKS) k_kbc_step(const KbcArgs a) {
@@ -702,24 +1109,108 @@ __global__ void __launch_bounds__(kThreads, FAST ? KBC_FAST_MIN_BLOCKS : KBC_MIN
   const uint32_t solid_mask =
       (EDGES && a.cmask && (a.bflags[b] & kNearSolid)) ? a.cmask[(int64_t)a.mslot[b] * 512 + cell] : 0u;
 
+  // the previous velocities of the six face neighbours (the WALE stencil, physics_utils.jl:2217-2233)
+  // and the cached multipliers; the fast path issues these loads before the pull, so that one trip to
+  // memory covers all three
+  float up[3][3], um[3][3];
+  auto load_velocities = [&]() {
+#pragma unroll
+    for (int ax = 0; ax < 3; ++ax) {
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        const int d = s == 0 ? 1 : -1;
+        const int px = x + (ax == 0 ? d : 0), py = y + (ax == 1 ? d : 0), pz = z + (ax == 2 ? d : 0);
+        const int ox = px < 0 ? -1 : (px > 7 ? 1 : 0), oy = py < 0 ? -1 : (py > 7 ? 1 : 0), oz = pz < 0 ? -1 : (pz > 7 ? 1 : 0);
+        const int bo = s_nbr[(ox + 1) + 3 * (oy + 1) + 9 * (oz + 1)];
+        // a neighbour outside the domain (ghost block) or in a solid cell contributes the own
+        // velocity (physics_utils.jl:1981-2035); mask bit of the D3Q27 direction whose source it is
+        const int sbit = ax == 0 ? (s == 0 ? 12 : 14) : ax == 1 ? (s == 0 ? 10 : 16) : (s == 0 ? 4 : 22);
+        const bool own = EDGES && (bo >= a.nb || ((solid_mask >> sbit) & 1u));
+        const int64_t c = own ? ci : ((px & 7) | ((py & 7) << 3) | ((pz & 7) << 6)) + 512 * (int64_t)bo;
+#pragma unroll
+        for (int comp = 0; comp < 3; ++comp) (s == 0 ? up : um)[ax][comp] = a.vin[c + N * comp];
+      }
+    }
+  };
+  // STEP 3: WALE from the previous velocity (physics_utils.jl:2217-2233, :2588-2700)
+  float g11, g22, g33, S12, S13, S23;
+  float nu_eddy = 0.0f;
+  auto wale = [&]() {
+    float g[9];
+#pragma unroll
+    for (int comp = 0; comp < 3; ++comp)
+#pragma unroll
+      for (int ax = 0; ax < 3; ++ax) g[3 * comp + ax] = 0.5f * (up[ax][comp] - um[ax][comp]);
+    const float g12 = g[1], g13 = g[2], g21 = g[3], g23 = g[5], g31 = g[6], g32 = g[7];
+    g11 = g[0]; g22 = g[4]; g33 = g[8];
+    S12 = 0.5f * (g12 + g21); S13 = 0.5f * (g13 + g31); S23 = 0.5f * (g23 + g32);
+    const float q11 = g11 * g11 + g12 * g21 + g13 * g31, q12 = g11 * g12 + g12 * g22 + g13 * g32, q13 = g11 * g13 + g12 * g23 + g13 * g33;
+    const float q21 = g21 * g11 + g22 * g21 + g23 * g31, q22 = g21 * g12 + g22 * g22 + g23 * g32, q23 = g21 * g13 + g22 * g23 + g23 * g33;
+    const float q31 = g31 * g11 + g32 * g21 + g33 * g31, q32 = g31 * g12 + g32 * g22 + g33 * g32, q33 = g31 * g13 + g32 * g23 + g33 * g33;
+    const float tr = (q11 + q22 + q33) / 3.0f;
+    const float Sd11 = q11 - tr, Sd22 = q22 - tr, Sd33 = q33 - tr;
+    const float Sd12 = 0.5f * (q12 + q21), Sd13 = 0.5f * (q13 + q31), Sd23 = 0.5f * (q23 + q32);
+    const float OP1 = Sd11 * Sd11 + Sd22 * Sd22 + Sd33 * Sd33 + 2.0f * (Sd12 * Sd12 + Sd13 * Sd13 + Sd23 * Sd23);
+    const float OP2 = g11 * g11 + g22 * g22 + g33 * g33 + 2.0f * (S12 * S12 + S13 * S13 + S23 * S23);
+    if (OP1 > 1e-12f) {
+      const float OP1_32 = OP1 * sqrtf(OP1);
+      const float OP2_52 = OP2 * OP2 * sqrtf(jmax(OP2, 1e-12f));
+      const float denom = OP2_52 + OP1 * sqrtf(sqrtf(jmax(OP1, 1e-12f)));
+      if (denom > 1e-12f) nu_eddy = (a.c_wale * a.c_wale) * OP1_32 / denom;
+    }
+  };
+  Eq<FAST> eq;
+  float* lam = a.lam + (int64_t)b * 13 * 512 + cell;
+  if constexpr (FAST) {
+    load_velocities();
+#pragma unroll
+    for (int m = 0; m < 13; ++m) eq.la[m] = lam[m * 512];
+  }
+
   // STEP 1-2: pull, moments, density floor and NaN reset (:898-1290, 1616-1650)
   float rho, ux, uy, uz, inv_rho;
+  float f_low = F_FLOOR;     // fast path: the smallest arriving population (at most the floor) ...
+  bool replaced = false;     // ... unless they were replaced after the pull
+  bool unbalanced = false;   // populations and macros may differ in mass or momentum
   {
     float jx = 0.0f, jy = 0.0f, jz = 0.0f;
     rho = 0.0f;
+    if constexpr (FAST) {
+      // unrolled: the offsets of the 39 pulls share the few shifted coordinates of each axis. All loads
+      // come before the first store to the column: the compiler cannot tell the two apart, and one
+      // trip to memory per direction was most of the kernel's time
+      float v[Q];
+#pragma unroll
+      for (int k = 0; k < Q; ++k) {
+        const int sx = x - kcx(k), sy = y - kcy(k), sz = z - kcz(k);
+        const int bo = s_nbr[(sx >> 3) + 3 * (sy >> 3) + 9 * (sz >> 3) + 13];
+        v[k] = (a.fin + (int64_t)bo * (Q * 512) + ((sx & 7) | ((sy & 7) << 3) | ((sz & 7) << 6)))[k * 512];
+      }
+#pragma unroll
+      for (int k = 0; k < Q; ++k) {
+        const float f = v[k];
+        sf[k * kThreads] = f;
+        f_low = fminf(f_low, f);
+        rho += f;
+        jx += f * float(kcx(k));
+        jy += f * float(kcy(k));
+        jz += f * float(kcz(k));
+      }
+    } else {
 #pragma unroll 13
-    for (int k = 0; k < Q; ++k) {
-      const int c = T.c[k];
-      const int cx = (c & 15) - 3, cy = ((c >> 4) & 15) - 3, cz = ((c >> 8) & 15) - 3;
-      const int sx = x - cx, sy = y - cy, sz = z - cz;
-      const int ox = sx < 0 ? -1 : (sx > 7 ? 1 : 0), oy = sy < 0 ? -1 : (sy > 7 ? 1 : 0), oz = sz < 0 ? -1 : (sz > 7 ? 1 : 0);
-      const int bo = s_nbr[(ox + 1) + 3 * (oy + 1) + 9 * (oz + 1)];
-      const float f = a.fin[((int64_t)bo * Q + k) * 512 + ((sx & 7) | ((sy & 7) << 3) | ((sz & 7) << 6))];
-      sf[k * kThreads] = f;
-      rho += f;
-      jx += f * float(cx);
-      jy += f * float(cy);
-      jz += f * float(cz);
+      for (int k = 0; k < Q; ++k) {
+        const int c = T.c[k];
+        const int cx = (c & 15) - 3, cy = ((c >> 4) & 15) - 3, cz = ((c >> 8) & 15) - 3;
+        const int sx = x - cx, sy = y - cy, sz = z - cz;
+        const int ox = sx < 0 ? -1 : (sx > 7 ? 1 : 0), oy = sy < 0 ? -1 : (sy > 7 ? 1 : 0), oz = sz < 0 ? -1 : (sz > 7 ? 1 : 0);
+        const int bo = s_nbr[(ox + 1) + 3 * (oy + 1) + 9 * (oz + 1)];
+        const float f = a.fin[((int64_t)bo * Q + k) * 512 + ((sx & 7) | ((sy & 7) << 3) | ((sz & 7) << 6))];
+        sf[k * kThreads] = f;
+        rho += f;
+        jx += f * float(cx);
+        jy += f * float(cy);
+        jz += f * float(cz);
+      }
     }
     if (EDGES && (solid_mask & (1u << 13))) {
       // simple bounce-back inside the obstacle (:1602-1613); the multiplier cache is left as it is
@@ -733,6 +1224,7 @@ __global__ void __launch_bounds__(kThreads, FAST ? KBC_FAST_MIN_BLOCKS : KBC_MIN
       // a cell on the inlet face (global x = 1): mass and momentum pinned to the inlet
       // equilibrium's (:1313-1352), then the moments again
       kbc::four_moment_pin(sf, kThreads, a.trho, a.tjx, a.tjy, a.tjz);
+      replaced = true;
       rho = 0.0f; jx = 0.0f; jy = 0.0f; jz = 0.0f;
 #pragma unroll 1
       for (int k = 0; k < Q; ++k) {
@@ -750,13 +1242,22 @@ __global__ void __launch_bounds__(kThreads, FAST ? KBC_FAST_MIN_BLOCKS : KBC_MIN
     const bool is_nan = !(rho_raw == rho_raw) || !(ux == ux) || !(uy == uy) || !(uz == uz);
     if (is_nan || rho_raw < 0.01f) {
       rho = 1.0f; ux = a.u_inlet; uy = 0.0f; uz = 0.0f; inv_rho = 1.0f;
+      replaced = unbalanced = true;
 #pragma unroll 1
       for (int k = 0; k < Q; ++k) sf[k * kThreads] = a.feq_inlet[k];
     }
   }
+  if constexpr (FAST) {
+    // the strain rates wait in the (still unused) h column for the HRR blend, where it is on
+    wale();
+    const float g[6] = {g11, g22, g33, S12, S13, S23};
+#pragma unroll
+    for (int i = 0; i < 6; ++i) sh[i * kThreads] = g[i];
+  }
   // sponge (kernel_entropic_d3q39.jl:1662, 1787-1841; athermal, pre-collision form)
   const float sp = a.sponge ? a.sponge[ci] : 0.0f;
   if (sp > 0.0f) {
+    replaced = unbalanced = true;
     rho = rho * (1.0f - sp) + 1.0f * sp;
     ux = ux * (1.0f - sp) + a.u_inlet * sp;
     uy = uy * (1.0f - sp);
@@ -840,64 +1341,29 @@ __global__ void __launch_bounds__(kThreads, FAST ? KBC_FAST_MIN_BLOCKS : KBC_MIN
   a.vout[ci + N] = uy;
   a.vout[ci + 2 * N] = uz;
   // STEP 3a: multipliers (warm start from the cache) and the mass correction (:2330-2385)
-  Eq<FAST> eq;
   eq.rho = rho;
+  [[maybe_unused]] float fe[FAST ? Q : 1];  // fast path: the equilibrium before the mass correction
   {
-    float* lam = a.lam + (int64_t)b * 13 * 512 + cell;
+    if constexpr (!FAST) {
 #pragma unroll
-    for (int m = 0; m < 13; ++m) eq.la[m] = lam[m * 512];
-    solve_lambdas<FAST>(T, rho, ux_rel, uy_rel, uz_rel, eq.la, a.warm_gate);
+      for (int m = 0; m < 13; ++m) eq.la[m] = lam[m * 512];
+    }
+    solve_lambdas<FAST>(T, rho, ux_rel, uy_rel, uz_rel, eq.la, fe, a.warm_gate);
 #pragma unroll
     for (int m = 0; m < 13; ++m) lam[m * 512] = eq.la[m];
     float sum = 0.0f;
+    if constexpr (FAST) {
+#pragma unroll
+      for (int k = 0; k < Q; ++k) sum += fe[k];
+    } else {
 #pragma unroll 3
-    for (int k = 0; k < Q; ++k) sum += fi_row<FAST>(rho, eq.la, T.b[k]);
+      for (int k = 0; k < Q; ++k) sum += fi_row<FAST>(rho, eq.la, T.b[k]);
+    }
     eq.corr = sum > 1e-15f ? rho / sum : 1.0f;
   }
-  // STEP 3: WALE from the previous velocity (physics_utils.jl:2217-2233, :2588-2700)
-  float g11, g22, g33, S12, S13, S23;
-  float nu_eddy = 0.0f;
-  {
-    float g[9];
-    float up[3][3], um[3][3];
-#pragma unroll
-    for (int ax = 0; ax < 3; ++ax) {
-#pragma unroll
-      for (int s = 0; s < 2; ++s) {
-        const int d = s == 0 ? 1 : -1;
-        const int px = x + (ax == 0 ? d : 0), py = y + (ax == 1 ? d : 0), pz = z + (ax == 2 ? d : 0);
-        const int ox = px < 0 ? -1 : (px > 7 ? 1 : 0), oy = py < 0 ? -1 : (py > 7 ? 1 : 0), oz = pz < 0 ? -1 : (pz > 7 ? 1 : 0);
-        const int bo = s_nbr[(ox + 1) + 3 * (oy + 1) + 9 * (oz + 1)];
-        // a neighbour outside the domain (ghost block) or in a solid cell contributes the own
-        // velocity (physics_utils.jl:1981-2035); mask bit of the D3Q27 direction whose source it is
-        const int sbit = ax == 0 ? (s == 0 ? 12 : 14) : ax == 1 ? (s == 0 ? 10 : 16) : (s == 0 ? 4 : 22);
-        const bool own = EDGES && (bo >= a.nb || ((solid_mask >> sbit) & 1u));
-        const int64_t c = own ? ci : ((px & 7) | ((py & 7) << 3) | ((pz & 7) << 6)) + 512 * (int64_t)bo;
-#pragma unroll
-        for (int comp = 0; comp < 3; ++comp) (s == 0 ? up : um)[ax][comp] = a.vin[c + N * comp];
-      }
-    }
-#pragma unroll
-    for (int comp = 0; comp < 3; ++comp)
-#pragma unroll
-      for (int ax = 0; ax < 3; ++ax) g[3 * comp + ax] = 0.5f * (up[ax][comp] - um[ax][comp]);
-    const float g12 = g[1], g13 = g[2], g21 = g[3], g23 = g[5], g31 = g[6], g32 = g[7];
-    g11 = g[0]; g22 = g[4]; g33 = g[8];
-    S12 = 0.5f * (g12 + g21); S13 = 0.5f * (g13 + g31); S23 = 0.5f * (g23 + g32);
-    const float q11 = g11 * g11 + g12 * g21 + g13 * g31, q12 = g11 * g12 + g12 * g22 + g13 * g32, q13 = g11 * g13 + g12 * g23 + g13 * g33;
-    const float q21 = g21 * g11 + g22 * g21 + g23 * g31, q22 = g21 * g12 + g22 * g22 + g23 * g32, q23 = g21 * g13 + g22 * g23 + g23 * g33;
-    const float q31 = g31 * g11 + g32 * g21 + g33 * g31, q32 = g31 * g12 + g32 * g22 + g33 * g32, q33 = g31 * g13 + g32 * g23 + g33 * g33;
-    const float tr = (q11 + q22 + q33) / 3.0f;
-    const float Sd11 = q11 - tr, Sd22 = q22 - tr, Sd33 = q33 - tr;
-    const float Sd12 = 0.5f * (q12 + q21), Sd13 = 0.5f * (q13 + q31), Sd23 = 0.5f * (q23 + q32);
-    const float OP1 = Sd11 * Sd11 + Sd22 * Sd22 + Sd33 * Sd33 + 2.0f * (Sd12 * Sd12 + Sd13 * Sd13 + Sd23 * Sd23);
-    const float OP2 = g11 * g11 + g22 * g22 + g33 * g33 + 2.0f * (S12 * S12 + S13 * S13 + S23 * S23);
-    if (OP1 > 1e-12f) {
-      const float OP1_32 = OP1 * sqrtf(OP1);
-      const float OP2_52 = OP2 * OP2 * sqrtf(jmax(OP2, 1e-12f));
-      const float denom = OP2_52 + OP1 * sqrtf(sqrtf(jmax(OP1, 1e-12f)));
-      if (denom > 1e-12f) nu_eddy = (a.c_wale * a.c_wale) * OP1_32 / denom;
-    }
+  if constexpr (!FAST) {
+    load_velocities();
+    wale();
   }
   nu_eddy = jmax(nu_eddy, a.nu_bg * a.amr_sgs_scale);
   // Mach-pocket viscosity (:2777-2806), shock sensor off
@@ -927,16 +1393,24 @@ __global__ void __launch_bounds__(kThreads, FAST ? KBC_FAST_MIN_BLOCKS : KBC_MIN
   hr.on = a.hrr;
   hr.sigma = a.hrr_sigma;
   hr.oms = 1.0f - a.hrr_sigma;
-  {
+  if (FAST && hr.on) {
+    g11 = sh[0]; g22 = sh[kThreads]; g33 = sh[2 * kThreads];
+    S12 = sh[3 * kThreads]; S13 = sh[4 * kThreads]; S23 = sh[5 * kThreads];
+  }
+  if (!FAST || hr.on) {
     const float c = -2.0f * rho * CS2 * jmax(tau_eff - 0.5f, 0.0f);
     hr.pxx = c * g11; hr.pyy = c * g22; hr.pzz = c * g33; hr.pxy = c * S12; hr.pxz = c * S13; hr.pyz = c * S23;
   }
   // STEP 4b: positivity of the arriving populations (:2885-2906)
   {
-    bool any_negative = false;
+    bool any_negative = FAST && f_low < F_FLOOR;
+    if (!FAST || replaced) {
+      any_negative = false;
 #pragma unroll 13
-    for (int k = 0; k < Q; ++k) any_negative = any_negative || sf[k * kThreads] < F_FLOOR;
+      for (int k = 0; k < Q; ++k) any_negative = any_negative || sf[k * kThreads] < F_FLOOR;
+    }
     if (any_negative) {
+      unbalanced = true;
       float worst = 1.0f;
 #pragma unroll 1
       for (int k = 0; k < Q; ++k) {
@@ -988,65 +1462,141 @@ __global__ void __launch_bounds__(kThreads, FAST ? KBC_FAST_MIN_BLOCKS : KBC_MIN
       }
     }
   }
-  // entropy of the arriving populations (:55-62), formed whether or not the alpha search runs
-  float H_pre = 0.0f;
-#pragma unroll 3
-  for (int k = 0; k < Q; ++k) {
-    const float fk = maxc(sf[k * kThreads], F_FLOOR);
-    H_pre = kmad<FAST>(fk, safe_log<FAST>(FAST ? fk * T.b[k][3].y : fk / T.b[k][3].x), H_pre);
-  }
-  const float inv_2beta = 0.5f / jmax(beta, 0.01f);
-  float alpha = 2.0f;
-  bool alpha_done = false;
-  if (a.solver == 3) alpha_done = alpha_taylor<FAST>(T, sf, eq, h_scale, hr, beta, alpha);
-  // STEP 5: split per pair, a_k = f_eq_k + coeff_s s_k over f_k (:2962-3095)
-  const float coeff_s = 1.0f - 2.0f * beta;
-#pragma unroll 1
-  for (int k = 0; k < Q; ++k) {
-    const int ps = T.ps[k];
-    if (!(ps & 0x200)) continue;
-    const int kb = (T.c[k] >> 12) & 63;
-    const float fe = eq(T, k), feb = kb == k ? fe : eq(T, kb);
-    const float df = sf[k * kThreads] - fe, dfb = sf[kb * kThreads] - feb;
-    const float s = hrr_s(T, 0.5f * (df + dfb), k, hr);
-    sh[(ps & 0xff) * kThreads] = (0.5f * (df - dfb)) * h_scale;
-    sf[k * kThreads] = fe + coeff_s * s;
-    if (kb != k) sf[kb * kThreads] = feb + coeff_s * s;
-  }
-  float h_norm_sq = 0.0f;
-#pragma unroll 13
-  for (int k = 0; k < Q; ++k) {
-    const float hk = h_at(T, sh, k);
-    h_norm_sq += hk * hk;
-  }
-  // STEP 6: alpha (:3109-3150)
-  if (h_norm_sq > 1e-20f) {
-    if (a.solver == 1) { alpha = alpha_newton<FAST>(T, sf, sh, beta, H_pre); alpha_done = true; }
-    else if (a.solver == 2) {
-      float fn = 0.0f;
-#pragma unroll 1
-      for (int k = 0; k < Q; ++k) {
-        const float fe = eq(T, k);
-        fn += fe * fe;
+  bool post_done = false;  // the fast path's column holds the post-collision populations
+  if constexpr (FAST) {
+    if (a.solver == 0 && !hr.on) {
+      const float coeff_s = 1.0f - 2.0f * beta;
+#pragma unroll
+      for (int k = 0; k < Q; ++k) fe[k] *= eq.corr;
+      AlphaSeries A;
+      bool decided = false;
+      float alpha_f = 2.0f;
+      // the series needs populations with the cell's mass and momentum and an unscaled h
+      if (sigma == 0.0f && !(guard > 0.0f) && !unbalanced && !macro_limited && !eq_limited && A.admits(sf, fe)) {
+        A.gather(sf, fe);
+        decided = A.solve(eq.la, beta, alpha_f);
       }
-      alpha = jclamp(2.0f - 0.5f * (h_norm_sq / jmax(fn, 1e-15f)), inv_2beta, 4.0f);
-      alpha_done = true;
+      // a_k = f_eq_k + coeff_s s_k, h per pair, and where the series did not decide the entropy of
+      // the arriving populations
+      float hv[19], h_sq = 0.0f;
+      {
+        float H0 = entropy_term(sf[0], 0, 0.0f), H1 = 0.0f;
+        fe[0] = fe[0] + coeff_s * (sf[0] - fe[0]);
+#pragma unroll
+        for (int p = 0; p < 19; ++p) {
+          const int k = kpos(p), kb = kopp(k);
+          const float fk = sf[k * kThreads], fb = sf[kb * kThreads];
+          if (!decided) {
+            H0 = entropy_term(fk, k, H0);
+            H1 = entropy_term(fb, kb, H1);
+          }
+          const float df = fk - fe[k], db = fb - fe[kb];
+          const float s = coeff_s * (0.5f * (df + db));
+          hv[p] = (0.5f * (df - db)) * h_scale;
+          fe[k] = fe[k] + s;
+          fe[kb] = fe[kb] + s;
+          h_sq = __fmaf_rn(2.0f * hv[p], hv[p], h_sq);
+        }
+        if (!decided) {
+          if (h_sq > 1e-20f) {
+            const float inv_2beta = 0.5f / fmaxf(beta, 0.01f);
+            alpha_f = alpha_bisection_regs(fe, hv, beta, H0 + H1);
+            if (!(alpha_f > 0.0f)) alpha_f = inv_2beta;
+            alpha_f = jclamp(alpha_f, inv_2beta, 6.0f);
+          } else {
+            alpha_f = 2.0f;
+          }
+        }
+      }
+      // KBC update; every population and their sum checked before the store
+      const float coeff = 1.0f - 2.0f * beta * alpha_f;
+      float low = fe[0], total = fe[0];
+#pragma unroll
+      for (int p = 0; p < 19; ++p) {
+        const int k = kpos(p), kb = kopp(k);
+        fe[k] = __fmaf_rn(coeff, hv[p], fe[k]);
+        fe[kb] = __fmaf_rn(-coeff, hv[p], fe[kb]);
+        low = fminf(low, fminf(fe[k], fe[kb]));
+        total += fe[k] + fe[kb];
+      }
+      if (!SVV && !(guard > 0.0f) && low >= 0.0f && total <= 1e3f) {  // nothing below zero, above 1e3 or NaN
+        float* fo = a.fout + (int64_t)b * Q * 512 + cell;
+#pragma unroll
+        for (int k = 0; k < Q; ++k) fo[k * 512] = fe[k];
+        return;
+      }
+#pragma unroll
+      for (int k = 0; k < Q; ++k) sf[k * kThreads] = fe[k];
+      post_done = true;
     }
-    if (!alpha_done) alpha = alpha_bisection<FAST>(T, sf, sh, beta, H_pre, 10);
-    if (!(alpha > 0.0f)) alpha = inv_2beta;
-    alpha = jclamp(alpha, inv_2beta, 6.0f);
-  } else {
-    alpha = 2.0f;
+  }
+  float coeff_h = 0.0f;
+  if (!post_done) {
+    // entropy of the arriving populations (:55-62), formed whether or not the alpha search runs
+    float H_pre = 0.0f;
+#pragma unroll 3
+    for (int k = 0; k < Q; ++k) {
+      const float fk = maxc(sf[k * kThreads], F_FLOOR);
+      H_pre = kmad<FAST>(fk, safe_log<FAST>(FAST ? fk * T.b[k][3].y : fk / T.b[k][3].x), H_pre);
+    }
+    const float inv_2beta = 0.5f / jmax(beta, 0.01f);
+    float alpha = 2.0f;
+    bool alpha_done = false;
+    if (a.solver == 3) alpha_done = alpha_taylor<FAST>(T, sf, eq, h_scale, hr, beta, alpha);
+    // STEP 5: split per pair, a_k = f_eq_k + coeff_s s_k over f_k (:2962-3095)
+    const float coeff_s = 1.0f - 2.0f * beta;
+#pragma unroll 1
+    for (int k = 0; k < Q; ++k) {
+      const int ps = T.ps[k];
+      if (!(ps & 0x200)) continue;
+      const int kb = (T.c[k] >> 12) & 63;
+      const float fe = eq(T, k), feb = kb == k ? fe : eq(T, kb);
+      const float df = sf[k * kThreads] - fe, dfb = sf[kb * kThreads] - feb;
+      const float s = hrr_s(T, 0.5f * (df + dfb), k, hr);
+      sh[(ps & 0xff) * kThreads] = (0.5f * (df - dfb)) * h_scale;
+      sf[k * kThreads] = fe + coeff_s * s;
+      if (kb != k) sf[kb * kThreads] = feb + coeff_s * s;
+    }
+    float h_norm_sq = 0.0f;
+#pragma unroll 13
+    for (int k = 0; k < Q; ++k) {
+      const float hk = h_at(T, sh, k);
+      h_norm_sq += hk * hk;
+    }
+    // STEP 6: alpha (:3109-3150)
+    if (h_norm_sq > 1e-20f) {
+      if (a.solver == 1) { alpha = alpha_newton<FAST>(T, sf, sh, beta, H_pre); alpha_done = true; }
+      else if (a.solver == 2) {
+        float fn = 0.0f;
+#pragma unroll 1
+        for (int k = 0; k < Q; ++k) {
+          const float fe = eq(T, k);
+          fn += fe * fe;
+        }
+        alpha = jclamp(2.0f - 0.5f * (h_norm_sq / jmax(fn, 1e-15f)), inv_2beta, 4.0f);
+        alpha_done = true;
+      }
+      if (!alpha_done) alpha = alpha_bisection<FAST>(T, sf, sh, beta, H_pre, 10);
+      if (!(alpha > 0.0f)) alpha = inv_2beta;
+      alpha = jclamp(alpha, inv_2beta, 6.0f);
+    } else {
+      alpha = 2.0f;
+    }
+    coeff_h = 1.0f - 2.0f * beta * alpha;
   }
   // STEP 7-8: KBC, post-collision blend and guard, output (:3153-3368). The zero body force adds
   // +-0 to a sum whose f_eq term is positive, which leaves it unchanged.
-  const float coeff_h = 1.0f - 2.0f * beta * alpha;
   float fmin = 1.0f;
+  if (post_done) {
 #pragma unroll 13
-  for (int k = 0; k < Q; ++k) {
-    const float v = sf[k * kThreads] + coeff_h * h_at(T, sh, k);
-    sf[k * kThreads] = v;
-    fmin = jmin(fmin, v);
+    for (int k = 0; k < Q; ++k) fmin = jmin(fmin, sf[k * kThreads]);
+  } else {
+#pragma unroll 13
+    for (int k = 0; k < Q; ++k) {
+      const float v = sf[k * kThreads] + coeff_h * h_at(T, sh, k);
+      sf[k * kThreads] = v;
+      fmin = jmin(fmin, v);
+    }
   }
   if (fmin < 0.0f) {
     float blend = 1.0f;
@@ -1131,7 +1681,8 @@ __global__ void __launch_bounds__(kThreads) k_kbc_init(const float* rho_in, cons
   Eq<> eq;
   eq.rho = r;
   eq.la[0] = qnan();
-  solve_lambdas(T, r, ux, uy, uz, eq.la);
+  float fe[1];
+  solve_lambdas(T, r, ux, uy, uz, eq.la, fe);
   float sum = 0.0f;
   for (int k = 0; k < Q; ++k) sum += fi_row(r, eq.la, T.b[k]);
   eq.corr = sum > 1e-15f ? r / sum : 1.0f;
