@@ -119,15 +119,23 @@ struct ParentView {
   // directions. Null: evaluate nodes on the fly.
   const int32_t* node_map;
   const void* node_vals;
-  // interpolation positions (the level's ghost cells whose pulls interpolate): slot_pos[(ghost
-  // block - real blocks) * 512 + cell] = position or -1; pos_nodes[position * 64 + 16(a+1) +
-  // 4(b+1) + (c+1)] = record of parent node (px0+a, py0+b, pz0+c) or -1 (absent); pos_macro =
-  // the interpolated rho, ux, uy, uz of each position (k_parent_positions, once per substep)
-  const int32_t* slot_pos;
-  const int32_t* pos_nodes;
-  const void* pos_macro;
-  int32_t n_pos, n_real;
+  const int32_t* nodes;  // [n_nodes] the parent cells of the records
+  int32_t n_nodes;
+  // interpolation groups (k_parent_fill): the ghost cells whose pulls interpolate, 2 x 2 x 2 fine
+  // cells (one parent bracket, one 4 x 4 x 4 stencil) per group. grp_xyz = (fx >> 1, fy >> 1, fz >> 1,
+  // GroupFlags) of the fine coordinates; grp_nodes[group * 64 + 16 (a + 1) + 4 (b + 1) + (c + 1)] =
+  // record of parent node (px0 + a, py0 + b, pz0 + c) or -1 (absent); grp_mem[group * 8 + ix + 2 iy +
+  // 4 iz] = (ghost slot = ghost block * 512 + cell, directions pulled from it), no directions = none.
+  // Null: every interpolated pull goes through the general fill.
+  const int4* grp_xyz;
+  const int32_t* grp_nodes;
+  const uint2* grp_mem;
+  int32_t n_groups;
+  // the level's other fill entries (domain faces, slip images)
+  const uint2* rest;
+  int64_t n_rest;
 };
+enum GroupFlags : int32_t { GF_CUBIC = 1, GF_ALL_NODES = 2 };
 
 // Restriction of a child level onto its parent (block AMR)
 struct RestrictArgs {

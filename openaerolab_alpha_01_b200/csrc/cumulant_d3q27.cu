@@ -39,19 +39,6 @@
 #ifndef OAL_FAST_CELLS
 #define OAL_FAST_CELLS 2
 #endif
-// refined levels' ghost fill: resident CTAs per SM its registers are sized for, and whether the
-// interpolation at a precomputed position is inlined
-#ifndef OAL_PAR_FILL_MIN_CTAS
-#define OAL_PAR_FILL_MIN_CTAS 4
-#endif
-#ifndef OAL_POS_NOINLINE
-#define OAL_POS_NOINLINE 0
-#endif
-#if OAL_POS_NOINLINE
-#define OAL_POS_LINKAGE __noinline__
-#else
-#define OAL_POS_LINKAGE
-#endif
 // threads per CTA of the x-pair kernel, one warp per z plane of a block: 32, 64, 128 or 256
 // (measured on the config-2 channel: 64 best, 128 1 % slower, 32 2 %, 256 12 %)
 #ifndef OAL_PAIRS_THREADS
@@ -190,27 +177,44 @@ __device__ __forceinline__ PNode<R> parent_macro(const ParentView& P, int pgx, i
 }
 
 // One thread per needed parent node: its time-blended macros and the f_neq of the 27 directions,
-// the same expressions the interpolation evaluates per stencil node
+// the same expressions the interpolation evaluates per stencil node. Each warp turns its 32 records
+// around in shared memory and writes them as whole 128-byte lines (one 4-byte store per thread and
+// value touched 32 lines each: 65 us a substep of the two-level sphere channel).
+constexpr int kNodeThreads = 64;
 template <class S, class R>
-__global__ void __launch_bounds__(256) k_parent_nodes(const ParentView P, const int32_t* __restrict__ nodes, int32_t n,
-                                                      R* __restrict__ vals, int32_t comp) {
-  const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int64_t c = nodes[i];
-  R* v = vals + (int64_t)i * 32;
-  const PNode<R> m = parent_macro_at<R>(P, c);
-  v[0] = m.rho; v[1] = m.ux; v[2] = m.uy; v[3] = m.uz;
+__global__ void __launch_bounds__(kNodeThreads) k_parent_nodes(const ParentView P, const int32_t* __restrict__ nodes,
+                                                               int32_t n, R* __restrict__ vals, int32_t comp) {
+  __shared__ R s_rec[kNodeThreads][33];
+  const int32_t base = blockIdx.x * kNodeThreads + (threadIdx.x & ~31), lane = threadIdx.x & 31;
+  const int32_t i = base + lane;
+  if (i < n) {
+    const int64_t c = nodes[i];
+    R* v = s_rec[threadIdx.x];
+    const PNode<R> m = parent_macro_at<R>(P, c);
+    v[0] = m.rho; v[1] = m.ux; v[2] = m.uy; v[3] = m.uz;
+    const int64_t fi = (c >> 9) * (27 * kCells) + (c & 511);
+    const S* fn = static_cast<const S*>(P.f_new) + fi;
+    const S* fo = static_cast<const S*>(P.f_old) + fi;
+    const bool blend = P.use_temporal == 1 && R(P.tw) < R(0.99) && P.f_old;
+    const R tw = R(P.tw);
 #pragma unroll
-  for (int k = 0; k < kQ27; ++k)
-    v[4 + k] = parent_blended_at<S, R>(P, c, k, R(q27_w(k)), R(q27_cx(k)), R(q27_cy(k)), R(q27_cz(k)), comp != 0).fneq;
-  v[31] = R(0);
+    for (int k = 0; k < kQ27; ++k) {
+      R f = Codec<S>::dec(fn[k * kCells], R(q27_w(k)), R(1.0 / q27_w(k)));
+      if (blend) f = Codec<S>::dec(fo[k * kCells], R(q27_w(k)), R(1.0 / q27_w(k))) * (R(1) - tw) + f * tw;
+      v[4 + k] = f - feq_c<R>(m.rho, m.ux, m.uy, m.uz, R(q27_w(k)), R(q27_cx(k)), R(q27_cy(k)), R(q27_cz(k)), comp != 0);
+    }
+    v[31] = R(0);
+  }
+  __syncwarp();
+  for (int j = 0; j < 32 && base + j < n; ++j) vals[(int64_t)(base + j) * 32 + lane] = s_rec[(threadIdx.x & ~31) + j][lane];
 }
 
 template <class S, class R>
-cudaError_t launch_parent_nodes(const ParentView& P, const int32_t* nodes, int32_t n, void* vals, int32_t comp,
-                                cudaStream_t st) {
-  if (n <= 0) return cudaSuccess;
-  k_parent_nodes<S, R><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(P, nodes, n, static_cast<R*>(vals), comp);
+cudaError_t launch_parent_nodes(const StepArgs& a, cudaStream_t st) {
+  const ParentView& P = a.par;
+  if (P.n_nodes <= 0) return cudaSuccess;
+  k_parent_nodes<S, R><<<(unsigned)((P.n_nodes + kNodeThreads - 1) / kNodeThreads), kNodeThreads, 0, st>>>(
+      P, P.nodes, P.n_nodes, static_cast<R*>(const_cast<void*>(P.node_vals)), (a.p0.flags & CF_COMPRESSIBLE) != 0);
   return cudaGetLastError();
 }
 
@@ -285,53 +289,34 @@ __device__ bool parent_sample_macro(const ParentView& P, int fgx, int fgy, int f
   return true;
 }
 
-// ---- interpolation at a precomputed position: the same arithmetic as parent_population below,
-// with the stencil's node records listed per position and its macros evaluated once per substep
+// ---- interpolation of the ghost cells from the node records (k_parent_fill) ----------------------
 template <class R>
-__device__ __forceinline__ void pos_record(const ParentView& P, const int32_t* nodes, int a, int b, int c,
-                                           bool& ok, const R*& v) {
+__device__ __forceinline__ void node_record(const R* vals, const int32_t* nodes, int a, int b, int c, bool& ok,
+                                            const R*& v) {
   const int32_t i = nodes[16 * (a + 1) + 4 * (b + 1) + (c + 1)];
   ok = i >= 0;
-  v = static_cast<const R*>(P.node_vals) + (int64_t)(ok ? i : 0) * 32;
+  v = vals + (int64_t)(ok ? i : 0) * 32;
 }
 
-// interpolated macros of a position (the macro half of interpolate_with_rescaling, :924-1129)
+// interpolated macros of a fine cell (the macro half of interpolate_with_rescaling, :924-1129) whose
+// stencil lacks a node or lies at the edge of the parent level
 template <class R>
-__device__ void pos_macros(const ParentView& P, int32_t pos, int fgx, int fgy, int fgz, R* out) {
-  const int32_t* nodes = P.pos_nodes + (int64_t)pos * 64;
-  const int pnx = P.dim_x * kBS, pny = P.dim_y * kBS, pnz = P.dim_z * kBS;
+__device__ __noinline__ void node_macros(const R* vals, int pnx, int pny, int pnz, const int32_t* nodes, int fgx,
+                                         int fgy, int fgz, R* out) {
   int px0, px1, py0, py1, pz0, pz1;
   R wx, wy, wz;
   parent_bracket<R>(R(fgx) * R(0.5) + R(0.25), pnx, px0, px1, wx);
   parent_bracket<R>(R(fgy) * R(0.5) + R(0.25), pny, py0, py1, wy);
   parent_bracket<R>(R(fgz) * R(0.5) + R(0.25), pnz, pz0, pz1, wz);
-  const bool use_cubic = px0 - 2 >= 1 && px0 + 2 <= pnx && py0 - 2 >= 1 && py0 + 2 <= pny && pz0 - 2 >= 1 &&
-                         pz0 + 2 <= pnz;
-  bool all_valid = use_cubic;
-  if (use_cubic)
-    for (int i = 0; i < 64 && all_valid; ++i) all_valid = nodes[i] >= 0;
   R rho_i, ux_i, uy_i, uz_i;
-  if (all_valid) {
-    rho_i = ux_i = uy_i = uz_i = R(0);
-    const Lagrange4<R> lx(wx), ly(wy), lz(wz);
-#pragma unroll 4
-    for (int i = 0; i < 64; ++i) {
-      const int a = i >> 4, bb = (i >> 2) & 3, c = i & 3;
-      const R* v = static_cast<const R*>(P.node_vals) + (int64_t)nodes[i] * 32;
-      const R w3 = lx.v[a] * ly.v[bb] * lz.v[c];
-      rho_i += w3 * v[0];
-      ux_i += w3 * v[1];
-      uy_i += w3 * v[2];
-      uz_i += w3 * v[3];
-    }
-  } else {
+  {
     // sample_parent_macro_for_fine_cell on the stencil's corner records (far nodes a, b, c = -1 or 2)
     PNode<R> d[8];
 #pragma unroll
     for (int cc = 0; cc < 8; ++cc) {
       bool ok;
       const R* v;
-      pos_record<R>(P, nodes, cc & 1, (cc >> 1) & 1, (cc >> 2) & 1, ok, v);
+      node_record<R>(vals, nodes, cc & 1, (cc >> 1) & 1, (cc >> 2) & 1, ok, v);
       d[cc] = ok ? PNode<R>{R(0), v[0], v[1], v[2], v[3], R(0), true} : PNode<R>{R(0), R(1), R(0), R(0), R(0), R(0), false};
     }
     const R w[8] = {(R(1) - wx) * (R(1) - wy) * (R(1) - wz), wx * (R(1) - wy) * (R(1) - wz),
@@ -359,7 +344,7 @@ __device__ void pos_macros(const ParentView& P, int32_t pos, int fgx, int fgy, i
           else ic = d[a].ok ? -1 : 2;
           bool fok;
           const R* fv;
-          pos_record<R>(P, nodes, ia, ib, ic, fok, fv);
+          node_record<R>(vals, nodes, ia, ib, ic, fok, fv);
           const PNode<R> s0 = d[src];
           d[dst].rho = fok ? R(2) * s0.rho - fv[0] : s0.rho;
           d[dst].ux = fok ? R(2) * s0.ux - fv[1] : s0.ux;
@@ -389,74 +374,9 @@ __device__ void pos_macros(const ParentView& P, int32_t pos, int fgx, int fgy, i
   out[0] = rho_i; out[1] = ux_i; out[2] = uy_i; out[3] = uz_i;
 }
 
-// One thread per interpolation position of the level: its interpolated macros for this substep
+// the rescaling of the interpolated f_neq (:1131-1198)
 template <class R>
-__global__ void __launch_bounds__(256) k_parent_positions(const ParentView P, const int4* __restrict__ pos_xyz,
-                                                          int32_t n, R* __restrict__ macro) {
-  const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int4 q = pos_xyz[i];
-  pos_macros<R>(P, i, q.x, q.y, q.z, macro + (int64_t)i * 4);
-}
-
-template <class R>
-cudaError_t launch_parent_positions(const ParentView& P, const int4* pos_xyz, int32_t n, void* macro, cudaStream_t st) {
-  if (n <= 0) return cudaSuccess;
-  k_parent_positions<R><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(P, pos_xyz, n, static_cast<R*>(macro));
-  return cudaGetLastError();
-}
-
-// the direction-dependent half at a position: f_neq over the stencil's records, then
-// feq(interpolated macros) + f_neq * scale (:1131-1198)
-template <class R>
-__device__ OAL_POS_LINKAGE R pos_population(const ParentView& P, int32_t pos, int fgx, int fgy, int fgz, int k, R cx, R cy, R cz,
-                            bool comp) {
-  const int32_t* nodes = P.pos_nodes + (int64_t)pos * 64;
-  const R* mac = static_cast<const R*>(P.pos_macro) + (int64_t)pos * 4;
-  const R wk = R(q27_w(k));
-  const int pnx = P.dim_x * kBS, pny = P.dim_y * kBS, pnz = P.dim_z * kBS;
-  int px0, px1, py0, py1, pz0, pz1;
-  R wx, wy, wz;
-  parent_bracket<R>(R(fgx) * R(0.5) + R(0.25), pnx, px0, px1, wx);
-  parent_bracket<R>(R(fgy) * R(0.5) + R(0.25), pny, py0, py1, wy);
-  parent_bracket<R>(R(fgz) * R(0.5) + R(0.25), pnz, pz0, pz1, wz);
-  const bool use_cubic = px0 - 2 >= 1 && px0 + 2 <= pnx && py0 - 2 >= 1 && py0 + 2 <= pny && pz0 - 2 >= 1 &&
-                         pz0 + 2 <= pnz;
-  // corner records and the anchor (first existing corner in 000, 100, 010, 110, 001, ... order)
-  int32_t corner[8];
-#pragma unroll
-  for (int cc = 0; cc < 8; ++cc) corner[cc] = nodes[16 * ((cc & 1) + 1) + 4 * (((cc >> 1) & 1) + 1) + ((cc >> 2) & 1) + 1];
-  int anchor = 7;
-#pragma unroll
-  for (int cc = 6; cc >= 0; --cc)
-    if (corner[cc] >= 0) anchor = cc;
-  const R* vals = static_cast<const R*>(P.node_vals);
-  // absent corner of a present anchor: the anchor's f_neq; no corner present: 0 (parent_blended's
-  // absent node)
-  const R anchor_neq = corner[anchor] >= 0 ? vals[(int64_t)corner[anchor] * 32 + 4 + k] : R(0);
-  R f_neq = R(0);
-  if (use_cubic) {
-    const Lagrange4<R> lx(wx), ly(wy), lz(wz);
-#pragma unroll 4
-    for (int i = 0; i < 64; ++i) {
-      const int a = i >> 4, bb = (i >> 2) & 3, c = i & 3;
-      const int32_t ni = nodes[i];
-      const R nv = ni >= 0 ? vals[(int64_t)ni * 32 + 4 + k] : anchor_neq;
-      f_neq += lx.v[a] * ly.v[bb] * lz.v[c] * nv;
-    }
-  } else {
-    R v[8];
-#pragma unroll
-    for (int cc = 0; cc < 8; ++cc) v[cc] = corner[cc] >= 0 ? vals[(int64_t)corner[cc] * 32 + 4 + k] : anchor_neq;
-    const R c00 = v[0] * (R(1) - wx) + v[1] * wx;
-    const R c01 = v[4] * (R(1) - wx) + v[5] * wx;
-    const R c10 = v[2] * (R(1) - wx) + v[3] * wx;
-    const R c11 = v[6] * (R(1) - wx) + v[7] * wx;
-    const R c0 = c00 * (R(1) - wy) + c10 * wy;
-    const R c1 = c01 * (R(1) - wy) + c11 * wy;
-    f_neq = c0 * (R(1) - wz) + c1 * wz;
-  }
-  const R feq_i = feq_c<R>(mac[0], mac[1], mac[2], mac[3], wk, cx, cy, cz, comp);
+__device__ __forceinline__ R parent_scale(const ParentView& P) {
   const R tau_p = R(P.tau_parent), tau_f = R(P.tau_fine);
   const R tau_c = tau_p - R(0.5), tau_fm = tau_f - R(0.5);
   R scale = tau_c > R(1e-6) ? fmin(fmax(tau_fm / tau_c, R(0.01)), R(100)) : R(1);
@@ -464,7 +384,123 @@ __device__ OAL_POS_LINKAGE R pos_population(const ParentView& P, int32_t pos, in
   const R omega_c = R(1) / fmax(tau_p, R(0.500001)), omega_f = R(1) / fmax(tau_f, R(0.500001));
   const R one_m_wc = R(1) - omega_c, one_m_wf = R(1) - omega_f;
   if (fabs(one_m_wc) > R(1e-6)) scale = fmin(fmax(scale * (one_m_wf / one_m_wc), R(0.01)), R(100));
-  return feq_i + f_neq * scale;
+  return scale;
+}
+
+// One warp per group of 2 x 2 x 2 fine cells that share their parent bracket (p + 1/4 and p + 3/4 per
+// axis) and so their 64-node stencil. Lane l carries value l of every record (rho, u, the f_neq of the
+// 27 directions), so a node is one coalesced 128-byte read, read once for all eight cells and all
+// directions; the tensor product of the axes' weights is contracted axis by axis (two weights each),
+// 112 multiply-adds per lane for the eight results. The macros then come from lanes 0-3 by shuffles
+// and each direction's lane writes its population. Bound by the L2 reads of the records (8 KB per
+// group). It replaces one thread per (cell, direction) with 64 gathered reads each and a separate pass
+// for the macros: 290 + 124 us per substep of the two-level sphere channel (256 x 128 x 128, refined
+// box 96 x 64 x 64, FP16; 131,000 ghost cells).
+template <class S, class R>
+__global__ void __launch_bounds__(128) k_parent_fill(const ParentView P, S* __restrict__ f, int32_t n_real, bool comp) {
+  const int32_t g = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (g >= P.n_groups) return;
+  const int4 gx = P.grp_xyz[g];
+  const int32_t* nodes = P.grp_nodes + (int64_t)g * 64;
+  const R* __restrict__ vals = static_cast<const R*>(P.node_vals) + lane;
+  const bool cubic = (gx.w & GF_CUBIC) != 0, all = (gx.w & GF_ALL_NODES) != 0;
+  // per axis and parity of the fine coordinate: the weights of the four nodes
+  R L[3][2][4];
+#pragma unroll
+  for (int ax = 0; ax < 3; ++ax) {
+    const int h = ax == 0 ? gx.x : ax == 1 ? gx.y : gx.z;
+    const int n = (ax == 0 ? P.dim_x : ax == 1 ? P.dim_y : P.dim_z) * kBS;
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      int i0, i1;
+      R w;
+      parent_bracket<R>(R(2 * h + s) * R(0.5) + R(0.25), n, i0, i1, w);
+      if (cubic) {
+        const Lagrange4<R> l(w);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) L[ax][s][i] = l.v[i];
+      } else {
+        // trilinear between the bracket's corners
+        L[ax][s][0] = R(0); L[ax][s][1] = R(1) - w; L[ax][s][2] = w; L[ax][s][3] = R(0);
+      }
+    }
+  }
+  // an absent node counts as the first existing corner (order 000, 100, 010, 110, 001, ...), or 0
+  R anchor = R(0);
+  if (!all) {
+    int32_t an = -1;
+#pragma unroll
+    for (int cc = 7; cc >= 0; --cc) {
+      const int32_t i = nodes[16 * ((cc & 1) + 1) + 4 * (((cc >> 1) & 1) + 1) + ((cc >> 2) & 1) + 1];
+      an = i >= 0 ? i : an;
+    }
+    if (an >= 0) anchor = vals[(int64_t)an * 32];
+  }
+  R acc[2][2][2] = {};
+#pragma unroll
+  for (int a = 0; a < 4; ++a) {
+    R yz[2][2] = {};
+    R v[4][4];
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      const int4 q = reinterpret_cast<const int4*>(nodes)[4 * a + b];
+      const int32_t id[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        // outside the cubic range only the bracket's corners count
+        const bool outer = a == 0 || a == 3 || b == 0 || b == 3 || c == 0 || c == 3;
+        if (outer && !cubic) v[b][c] = R(0);
+        else v[b][c] = (all || id[c] >= 0) ? vals[(int64_t)id[c] * 32] : anchor;
+      }
+    }
+#pragma unroll
+    for (int b = 0; b < 4; ++b)
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        R z = L[2][s][0] * v[b][0];
+#pragma unroll
+        for (int c = 1; c < 4; ++c) z = vfma(L[2][s][c], v[b][c], z);
+        yz[0][s] = vfma(L[1][0][b], z, yz[0][s]);
+        yz[1][s] = vfma(L[1][1][b], z, yz[1][s]);
+      }
+#pragma unroll
+    for (int iy = 0; iy < 2; ++iy)
+#pragma unroll
+      for (int iz = 0; iz < 2; ++iz) {
+        acc[0][iy][iz] = vfma(L[0][0][a], yz[iy][iz], acc[0][iy][iz]);
+        acc[1][iy][iz] = vfma(L[0][1][a], yz[iy][iz], acc[1][iy][iz]);
+      }
+  }
+  const int k = lane >= 4 && lane < 31 ? lane - 4 : 0;
+  const int cxi = k % 3 - 1, cyi = (k / 3) % 3 - 1, czi = k / 9 - 1, d2 = cxi * cxi + cyi * cyi + czi * czi;
+  const R wk = d2 == 0 ? R(8.0 / 27.0) : d2 == 1 ? R(2.0 / 27.0) : d2 == 2 ? R(1.0 / 54.0) : R(1.0 / 216.0);
+  const R iwk = d2 == 0 ? R(27.0 / 8.0) : d2 == 1 ? R(13.5) : d2 == 2 ? R(54) : R(216);
+  const R scale = parent_scale<R>(P);
+  R own[4] = {R(1), R(0), R(0), R(0)};
+  if (!(cubic && all) && lane < 8 && P.grp_mem[(int64_t)g * 8 + lane].y != 0u)
+    node_macros<R>(static_cast<const R*>(P.node_vals), P.dim_x * kBS, P.dim_y * kBS, P.dim_z * kBS, nodes, 2 * gx.x + (lane & 1), 2 * gx.y + ((lane >> 1) & 1), 2 * gx.z + (lane >> 2), own);
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const uint2 m = P.grp_mem[(int64_t)g * 8 + j];
+    if (m.y == 0u) continue;
+    const R v = acc[j & 1][(j >> 1) & 1][j >> 2];
+    R mac[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      mac[i] = cubic && all ? __shfl_sync(0xffffffffu, v, i) : __shfl_sync(0xffffffffu, own[i], j);
+    if (lane >= 4 && ((m.y >> k) & 1u) && lane < 31) {
+      const R fe = feq_c<R>(mac[0], mac[1], mac[2], mac[3], wk, R(cxi), R(cyi), R(czi), comp);
+      f[((int64_t)(m.x >> 9) + n_real) * (27 * kCells) + k * kCells + (m.x & 511u)] = Codec<S>::enc(fe + v * scale, wk, iwk);
+    }
+  }
+}
+
+template <class S, class R>
+cudaError_t launch_parent_fill(const StepArgs& a, cudaStream_t st) {
+  if (a.par.n_groups <= 0) return cudaSuccess;
+  k_parent_fill<S, R><<<(unsigned)((a.par.n_groups + 3) / 4), 128, 0, st>>>(
+      a.par, const_cast<S*>(static_cast<const S*>(a.f_in)), a.n_blocks, (a.p0.flags & CF_COMPRESSIBLE) != 0);
+  return cudaGetLastError();
 }
 
 // interpolate_with_rescaling at the fine cell (fgx, fgy, fgz) of the refined level, direction k
@@ -539,14 +575,7 @@ __device__ __noinline__ R parent_population(const ParentView& P, int fgx, int fg
   } else {
     f_neq = trilin(&PNode<R>::fneq);
   }
-  const R tau_p = R(P.tau_parent), tau_f = R(P.tau_fine);
-  const R tau_c = tau_p - R(0.5), tau_fm = tau_f - R(0.5);
-  R scale = tau_c > R(1e-6) ? fmin(fmax(tau_fm / tau_c, R(0.01)), R(100)) : R(1);
-  if (P.level_visc_physical == 1) scale = fmin(fmax(tau_f / (R(2) * fmax(tau_p, R(0.500001))), R(0.01)), R(100));
-  const R omega_c = R(1) / fmax(tau_p, R(0.500001)), omega_f = R(1) / fmax(tau_f, R(0.500001));
-  const R one_m_wc = R(1) - omega_c, one_m_wf = R(1) - omega_f;
-  if (fabs(one_m_wc) > R(1e-6)) scale = fmin(fmax(scale * (one_m_wf / one_m_wc), R(0.01)), R(100));
-  return feq_i + f_neq * scale;
+  return feq_i + f_neq * parent_scale<R>(P);
 }
 
 // Population arriving at cell (x,y,z) of block b in direction k from outside every block
@@ -613,16 +642,7 @@ __device__ __forceinline__ R face_population_impl(const S* __restrict__ fin, int
   } else if (is_z_min || is_z_max) {
     j = q27_mir_z(k);
   } else if (PAR && da && da->par.ptr) {
-    // refined level: interpolated from the parent (kernel_cumulant.jl:346-388); the source is a
-    // ghost cell whose interpolation position may be precomputed
-    if (da->par.slot_pos && !DENSE) {
-      const int sx = x - cx, sy = y - cy, sz = z - cz;
-      const int g = nbr[nbr_dir(sx >> 3, sy >> 3, sz >> 3)];
-      if (g >= n_real) {
-        const int32_t pos = da->par.slot_pos[(int64_t)(g - n_real) * kCells + ((sx & 7) | ((sy & 7) << 3) | ((sz & 7) << 6))];
-        if (pos >= 0) return pos_population<R>(da->par, pos, src_gx, src_gy, src_gz, k, R(cx), R(cy), R(cz), comp);
-      }
-    }
+    // refined level: interpolated from the parent (kernel_cumulant.jl:346-388)
     return parent_population<S, R>(da->par, src_gx, src_gy, src_gz, k, R(cx), R(cy), R(cz), comp);
   } else {
     return R(q27_w(k));  // kernel_cumulant.jl:389-391
@@ -653,7 +673,7 @@ __device__ __forceinline__ const CaseParams& case_of(const StepArgs& a, int case
 // PAR: the level has a parent (its ghost pulls from inside the domain interpolate from it); the
 // plain instance carries none of that code and stays small
 template <class S, class R, bool DENSE, bool PAR>
-__global__ void __launch_bounds__(256, PAR ? OAL_PAR_FILL_MIN_CTAS : 1) k_fill_ghosts(const StepArgs a, const uint2* __restrict__ entries, int64_t n) {
+__global__ void __launch_bounds__(256) k_fill_ghosts(const StepArgs a, const uint2* __restrict__ entries, int64_t n) {
   const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (e >= n) return;
   const uint2 en = entries[e];
@@ -1813,8 +1833,8 @@ cudaError_t launch_general(const StepArgs& a, const int32_t* work, int n_work, c
   template cudaError_t launch_fill_ghosts<S, R>(const StepArgs&, const uint2*, int64_t, cudaStream_t); \
   template cudaError_t launch_fill_copy<S, R>(const StepArgs&, const uint2*, int64_t, cudaStream_t, bool); \
   template cudaError_t launch_restrict<S, R>(const RestrictArgs&, cudaStream_t);                       \
-  template cudaError_t launch_parent_nodes<S, R>(const ParentView&, const int32_t*, int32_t, void*, int32_t,  \
-                                                 cudaStream_t);                                            \
+  template cudaError_t launch_parent_nodes<S, R>(const StepArgs&, cudaStream_t);                       \
+  template cudaError_t launch_parent_fill<S, R>(const StepArgs&, cudaStream_t);                        \
   template cudaError_t launch_fast<S, R>(const StepArgs&, const int32_t*, int, cudaStream_t);         \
   template cudaError_t launch_general<S, R>(const StepArgs&, const int32_t*, int, cudaStream_t);
 OAL_INST(float, float)
@@ -1822,7 +1842,5 @@ OAL_INST(__half, float)
 OAL_INST(__nv_bfloat16, float)
 OAL_INST(double, double)
 #undef OAL_INST
-template cudaError_t launch_parent_positions<float>(const ParentView&, const int4*, int32_t, void*, cudaStream_t);
-template cudaError_t launch_parent_positions<double>(const ParentView&, const int4*, int32_t, void*, cudaStream_t);
 
 }  // namespace oal

@@ -7,6 +7,7 @@
 #include <cstring>
 #include <cmath>
 #include <string>
+#include <tuple>
 #include <vector>
 #include <algorithm>
 
@@ -36,10 +37,9 @@ int dense_ctas_per_sm();
 template <class S, class R>
 cudaError_t launch_restrict(const RestrictArgs& r, cudaStream_t st);
 template <class S, class R>
-cudaError_t launch_parent_nodes(const ParentView& P, const int32_t* nodes, int32_t n, void* vals, int32_t comp,
-                                cudaStream_t st);
-template <class R>
-cudaError_t launch_parent_positions(const ParentView& P, const int4* pos_xyz, int32_t n, void* macro, cudaStream_t st);
+cudaError_t launch_parent_nodes(const StepArgs& a, cudaStream_t st);
+template <class S, class R>
+cudaError_t launch_parent_fill(const StepArgs& a, cudaStream_t st);
 }
 using namespace oal;
 
@@ -698,6 +698,13 @@ static cudaError_t launch_step_t(const oal_geometry* g, const StepArgs& a0, Step
       if (c.key == fill_key_of(a.p0.flags)) fl = &c;
   auto fill = [&](cudaStream_t s) -> cudaError_t {
     cudaError_t r;
+    if (a.par.ptr) {
+      // refined level: the records of the parent nodes, the interpolated ghost cells, then the rest
+      // (domain faces and slip images, which read the records too)
+      if ((r = launch_parent_nodes<S, R>(a, s)) != cudaSuccess) return r;
+      if ((r = launch_parent_fill<S, R>(a, s)) != cudaSuccess) return r;
+      return launch_fill_ghosts<S, R>(a, a.par.rest, a.par.n_rest, s);
+    }
     if (!fl) return launch_fill_ghosts<S, R>(a, g->d_gentries, g->n_gentries, s);
     if ((r = launch_fill_copy<S, R>(a, fl->copy, fl->n_copy, s)) != cudaSuccess) return r;
     return launch_fill_ghosts<S, R>(a, fl->rest, fl->n_rest, s);
@@ -2159,20 +2166,23 @@ struct AmrLevel {
   int32_t* d_ptr = nullptr;       // block pointer [dim_x*dim_y*dim_z], x fastest, 1-based
   int32_t* d_covered = nullptr;   // this level's blocks that have children
   int32_t n_covered = 0;
-  void* d_f_old = nullptr;        // snapshot before the level's step (levels with children)
-  void* d_rho_old = nullptr;
-  void* d_vel_old = nullptr;
+  void* d_rho_old = nullptr;      // density before the level's step (levels with children)
   // refined levels: the parent nodes their interpolation stencils touch, evaluated once per substep
-  int32_t* d_nodes = nullptr;     // parent cell ids (block * 512 + cell)
+  int32_t* d_nodes = nullptr;     // parent cell ids (block * 512 + cell), ascending
   int32_t n_nodes = 0;
   int32_t* d_node_map = nullptr;  // [parent cells] -> record index, -1
   void* d_node_vals = nullptr;    // [n_nodes * 32] compute type
-  // interpolation positions: the ghost cells whose pulls interpolate from the parent
-  int32_t n_pos = 0;
-  int4* d_pos_xyz = nullptr;      // fine global coordinates of each position
-  int32_t* d_slot_pos = nullptr;  // [ghost blocks * 512] -> position, -1
-  int32_t* d_pos_nodes = nullptr; // [n_pos * 64] stencil records, -1 = absent parent cell
-  void* d_pos_macro = nullptr;    // [n_pos * 4] compute type
+  // interpolation groups and the other fill entries (ParentView)
+  int32_t n_groups = 0;
+  int4* d_grp_xyz = nullptr;
+  int32_t* d_grp_nodes = nullptr;
+  uint2* d_grp_mem = nullptr;
+  uint2* d_rest = nullptr;
+  int64_t n_rest = 0;
+  // populations and velocity before the level's step: the step's input buffers, which no launch of
+  // the coarse step rewrites (set by amr_step)
+  const void* f_old = nullptr;
+  const void* vel_old = nullptr;
 };
 
 struct oal_amr {
@@ -2213,23 +2223,26 @@ static oal_status amr_step(oal_amr* A, int l, const std::vector<CaseParams>& cps
   oal_level* L = me.L;
   const oal_geometry* g = me.g;
   const bool has_children = l + 1 < (int)A->lv.size();
-  const size_t sb = storage_bytes(A->storage), mb = macro_bytes(A->storage);
-  const size_t ncell = (size_t)g->nb * 512;
-  if (has_children) {  // copy_to_old! (src/geometry/blocks.jl:604-640)
+  const size_t mb = macro_bytes(A->storage), ncell = (size_t)g->nb * 512;
+  if (has_children) {
+    // copy_to_old! (src/geometry/blocks.jl:604-640): the step writes the other population and velocity
+    // buffer and nothing rewrites this one before the level's next step (its ghost fill touches ghost
+    // blocks only, the restriction the new buffer), so the old state is the input buffers themselves;
+    // only the density has one buffer
     const int p = L->parity;
-    OAL_CUDA_TRY(cudaMemcpyAsync(me.d_f_old, L->f[p], ncell * 27 * sb, cudaMemcpyDeviceToDevice, st));
+    me.f_old = L->f[p];
+    me.vel_old = L->vel[p];
     OAL_CUDA_TRY(cudaMemcpyAsync(me.d_rho_old, L->rho, ncell * mb, cudaMemcpyDeviceToDevice, st));
-    OAL_CUDA_TRY(cudaMemcpyAsync(me.d_vel_old, L->vel[p], ncell * 3 * mb, cudaMemcpyDeviceToDevice, st));
   }
   if (l > 0) {
     const AmrLevel& pa = A->lv[(size_t)l - 1];
     ParentView v{};
     v.f_new = pa.L->f[pa.L->parity];
-    v.f_old = pa.d_f_old;
+    v.f_old = pa.f_old;
     v.rho_new = pa.L->rho;
     v.rho_old = pa.d_rho_old;
     v.vel_new = pa.L->vel[pa.L->parity];
-    v.vel_old = pa.d_vel_old;
+    v.vel_old = pa.vel_old;
     v.ptr = pa.d_ptr;
     v.dim_x = pa.dim[0]; v.dim_y = pa.dim[1]; v.dim_z = pa.dim[2];
     v.nb = pa.g->nb;
@@ -2240,28 +2253,15 @@ static oal_status amr_step(oal_amr* A, int l, const std::vector<CaseParams>& cps
     v.level_visc_physical = P[l].level_visc_physical;
     v.node_map = me.d_node_map;
     v.node_vals = me.d_node_vals;
-    v.slot_pos = me.n_pos > 0 ? me.d_slot_pos : nullptr;
-    v.pos_nodes = me.d_pos_nodes;
-    v.pos_macro = me.d_pos_macro;
-    v.n_pos = me.n_pos;
-    v.n_real = me.g->nb;
+    v.nodes = me.d_nodes;
+    v.n_nodes = me.n_nodes;
+    v.grp_xyz = me.d_grp_xyz;
+    v.grp_nodes = me.d_grp_nodes;
+    v.grp_mem = me.d_grp_mem;
+    v.n_groups = me.n_groups;
+    v.rest = me.d_rest;
+    v.n_rest = me.n_rest;
     L->par = v;
-    if (me.n_nodes > 0) {
-      cudaError_t e = cudaErrorInvalidValue;
-      const int32_t comp = P[l].compressible_corr;
-      switch (A->storage) {
-        case OAL_STORE_F32: e = launch_parent_nodes<float, float>(v, me.d_nodes, me.n_nodes, me.d_node_vals, comp, st); break;
-        case OAL_STORE_F16_DEV: e = launch_parent_nodes<__half, float>(v, me.d_nodes, me.n_nodes, me.d_node_vals, comp, st); break;
-        case OAL_STORE_BF16_DEV: e = launch_parent_nodes<__nv_bfloat16, float>(v, me.d_nodes, me.n_nodes, me.d_node_vals, comp, st); break;
-        case OAL_STORE_F64: e = launch_parent_nodes<double, double>(v, me.d_nodes, me.n_nodes, me.d_node_vals, comp, st); break;
-      }
-      OAL_CUDA_TRY(e);
-      if (me.n_pos > 0) {
-        e = A->storage == OAL_STORE_F64 ? launch_parent_positions<double>(v, me.d_pos_xyz, me.n_pos, me.d_pos_macro, st)
-                                        : launch_parent_positions<float>(v, me.d_pos_xyz, me.n_pos, me.d_pos_macro, st);
-        OAL_CUDA_TRY(e);
-      }
-    }
   }
   CaseParams cp = cps[(size_t)l];
   cp.time_step_seed = (int32_t)(P[l].time_step_seed + t_sub);
@@ -2318,9 +2318,9 @@ void oal_amr_destroy(oal_amr* A) {
   amr_release_graph(A);
   for (AmrLevel& l : A->lv) {
     if (l.L) oal_level_destroy(l.L);
-    cudaFree(l.d_ptr); cudaFree(l.d_covered); cudaFree(l.d_f_old); cudaFree(l.d_rho_old); cudaFree(l.d_vel_old);
+    cudaFree(l.d_ptr); cudaFree(l.d_covered); cudaFree(l.d_rho_old);
     cudaFree(l.d_nodes); cudaFree(l.d_node_map); cudaFree(l.d_node_vals);
-    cudaFree(l.d_pos_xyz); cudaFree(l.d_slot_pos); cudaFree(l.d_pos_nodes); cudaFree(l.d_pos_macro);
+    cudaFree(l.d_grp_xyz); cudaFree(l.d_grp_nodes); cudaFree(l.d_grp_mem); cudaFree(l.d_rest);
   }
   if (A->cap) cudaStreamDestroy(A->cap);
   cudaGetLastError();
@@ -2410,9 +2410,7 @@ oal_status oal_amr_create(int32_t nlevels, const oal_amr_level_desc* levels, int
       if (e == cudaSuccess && !cov.empty())
         e = cudaMemcpy(me.d_covered, cov.data(), cov.size() * sizeof(int32_t), cudaMemcpyHostToDevice);
       const size_t ncell = (size_t)me.g->nb * 512;
-      if (e == cudaSuccess) e = cudaMalloc(&me.d_f_old, ncell * 27 * storage_bytes(storage));
       if (e == cudaSuccess) e = cudaMalloc(&me.d_rho_old, ncell * macro_bytes(storage));
-      if (e == cudaSuccess) e = cudaMalloc(&me.d_vel_old, ncell * 3 * macro_bytes(storage));
     }
     if (e == cudaSuccess && l > 0) {
       // parent nodes of every interpolation stencil this level's ghost pulls can use: the 4x4x4
@@ -2445,10 +2443,12 @@ oal_status oal_amr_create(int32_t nlevels, const oal_amr_level_desc* levels, int
               if (map[(size_t)cid] < 0) { map[(size_t)cid] = (int32_t)nodes.size(); nodes.push_back(cid); }
             }
       };
-      // interpolation positions: every ghost cell that an in-domain pull reads (its slot in the
-      // ghost blocks), with the record of each of its 64 stencil nodes
+      // every ghost cell that an in-domain pull reads (its slot in the ghost blocks): its fine
+      // coordinates and the directions pulled from it; the level's other entries
+      struct Pos { int32_t x, y, z, slot; uint32_t dirs; };
       std::vector<int32_t> slot_pos((size_t)std::max(g->n_ghost, 1) * 512, -1);
-      std::vector<int4> pos_xyz;
+      std::vector<Pos> pos;
+      std::vector<uint2> rest;
       for (const uint2& en : g->h_gentries) {
         const int4 bi = g->h_binfo[en.x];
         const int cell = (int)(en.y & 511u), k = (int)((en.y >> 9) & 31u);
@@ -2456,6 +2456,7 @@ oal_status oal_amr_create(int32_t nlevels, const oal_amr_level_desc* levels, int
         const int gx = (bi.x - 1) * 8 + x + 1, gy = (bi.y - 1) * 8 + y + 1, gz = (bi.z - 1) * 8 + z + 1;
         const int sx = gx - q27_cx(k), sy = gy - q27_cy(k), sz = gz - q27_cz(k);
         const bool in_x = sx >= 1 && sx <= g->nx, in_y = sy >= 1 && sy <= g->ny, in_z = sz >= 1 && sz <= g->nz;
+        bool grouped = false;
         if (in_x && in_y && in_z) {
           add_stencil(sx, sy, sz);
           const int lx = x - q27_cx(k), ly = y - q27_cy(k), lz = z - q27_cz(k);
@@ -2463,62 +2464,77 @@ oal_status oal_amr_create(int32_t nlevels, const oal_amr_level_desc* levels, int
                     oz = lz < 0 ? -1 : (lz > 7 ? 1 : 0);
           const int32_t gb = g->h_nbrg[(size_t)en.x * 27 + nbr_dir(ox, oy, oz)];
           if (gb >= g->nb && gb < g->nb + g->n_ghost) {
-            const size_t slot = (size_t)(gb - g->nb) * 512 + ((lx & 7) | ((ly & 7) << 3) | ((lz & 7) << 6));
-            if (slot_pos[slot] < 0) { slot_pos[slot] = (int32_t)pos_xyz.size(); pos_xyz.push_back(make_int4(sx, sy, sz, 0)); }
+            const int32_t slot = (gb - g->nb) * 512 + ((lx & 7) | ((ly & 7) << 3) | ((lz & 7) << 6));
+            int32_t& at = slot_pos[(size_t)slot];
+            if (at < 0) { at = (int32_t)pos.size(); pos.push_back(Pos{sx, sy, sz, slot, 0u}); }
+            // the slot's cell must be the pull's source cell (one ghost block per grid position)
+            if (pos[(size_t)at].x == sx && pos[(size_t)at].y == sy && pos[(size_t)at].z == sz) {
+              pos[(size_t)at].dirs |= 1u << k;
+              grouped = true;
+            }
           }
         } else if (in_x && in_y && !in_z) {
           add_stencil(sx, sy, gz);
         }
+        if (!grouped) rest.push_back(en);
       }
-      std::vector<int32_t> pos_nodes(pos_xyz.size() * 64, -1);
-      for (size_t i = 0; i < pos_xyz.size(); ++i) {
-        const int px0 = bracket(pos_xyz[i].x * 0.5 + 0.25, pnx), py0 = bracket(pos_xyz[i].y * 0.5 + 0.25, pny),
-                  pz0 = bracket(pos_xyz[i].z * 0.5 + 0.25, pnz);
-        for (int a = -1; a <= 2; ++a)
-          for (int b2 = -1; b2 <= 2; ++b2)
-            for (int c2 = -1; c2 <= 2; ++c2) {
-              const int gx = px0 + a, gy = py0 + b2, gz = pz0 + c2;
-              if (gx < 1 || gy < 1 || gz < 1) continue;
-              const int bx = (gx - 1) / 8 + 1, by = (gy - 1) / 8 + 1, bz = (gz - 1) / 8 + 1;
-              if (bx > pa.dim[0] || by > pa.dim[1] || bz > pa.dim[2]) continue;
-              const int32_t pb = pptr[(size_t)(bx - 1) + (size_t)pa.dim[0] * ((by - 1) + (size_t)pa.dim[1] * (bz - 1))];
-              if (pb <= 0) continue;
-              const int32_t cid = (pb - 1) * 512 + (((gx - 1) % 8) | (((gy - 1) % 8) << 3) | (((gz - 1) % 8) << 6));
-              pos_nodes[i * 64 + (size_t)(16 * (a + 1) + 4 * (b2 + 1) + (c2 + 1))] = map[(size_t)cid];
-            }
+      // records in the order of the parent's cells, so that neighbouring threads read neighbouring cells
+      std::sort(nodes.begin(), nodes.end());
+      for (size_t i = 0; i < nodes.size(); ++i) map[(size_t)nodes[i]] = (int32_t)i;
+      // groups of 2 x 2 x 2 fine cells in grid order; a second ghost slot of the same cell (two ghost
+      // blocks at one grid position) opens another group
+      std::stable_sort(pos.begin(), pos.end(), [](const Pos& a, const Pos& b) {
+        return std::make_tuple(a.z >> 1, a.y >> 1, a.x >> 1) < std::make_tuple(b.z >> 1, b.y >> 1, b.x >> 1);
+      });
+      std::vector<int4> grp_xyz;
+      std::vector<int32_t> grp_nodes;
+      std::vector<uint2> grp_mem;
+      for (const Pos& q : pos) {
+        const int j = (q.x & 1) + 2 * (q.y & 1) + 4 * (q.z & 1);
+        const int hx = q.x >> 1, hy = q.y >> 1, hz = q.z >> 1;
+        const bool same = !grp_xyz.empty() && grp_xyz.back().x == hx && grp_xyz.back().y == hy &&
+                          grp_xyz.back().z == hz && grp_mem[(grp_xyz.size() - 1) * 8 + (size_t)j].y == 0u;
+        if (!same) {
+          const int px0 = bracket(q.x * 0.5 + 0.25, pnx), py0 = bracket(q.y * 0.5 + 0.25, pny), pz0 = bracket(q.z * 0.5 + 0.25, pnz);
+          const bool cubic = px0 - 2 >= 1 && px0 + 2 <= pnx && py0 - 2 >= 1 && py0 + 2 <= pny && pz0 - 2 >= 1 && pz0 + 2 <= pnz;
+          bool all = true;
+          for (int a = -1; a <= 2; ++a)
+            for (int b2 = -1; b2 <= 2; ++b2)
+              for (int c2 = -1; c2 <= 2; ++c2) {
+                const int gx = px0 + a, gy = py0 + b2, gz = pz0 + c2;
+                int32_t rec = -1;
+                if (gx >= 1 && gy >= 1 && gz >= 1) {
+                  const int bx = (gx - 1) / 8 + 1, by = (gy - 1) / 8 + 1, bz = (gz - 1) / 8 + 1;
+                  if (bx <= pa.dim[0] && by <= pa.dim[1] && bz <= pa.dim[2]) {
+                    const int32_t pb = pptr[(size_t)(bx - 1) + (size_t)pa.dim[0] * ((by - 1) + (size_t)pa.dim[1] * (bz - 1))];
+                    if (pb > 0) rec = map[(size_t)((pb - 1) * 512 + (((gx - 1) % 8) | (((gy - 1) % 8) << 3) | (((gz - 1) % 8) << 6)))];
+                  }
+                }
+                all = all && rec >= 0;
+                grp_nodes.push_back(rec);
+              }
+          grp_xyz.push_back(make_int4(hx, hy, hz, (cubic ? GF_CUBIC : 0) | (all ? GF_ALL_NODES : 0)));
+          grp_mem.resize(grp_xyz.size() * 8, make_uint2(0u, 0u));
+        }
+        grp_mem[(grp_xyz.size() - 1) * 8 + (size_t)j] = make_uint2((uint32_t)q.slot, q.dirs);
       }
       me.n_nodes = (int32_t)nodes.size();
+      me.n_groups = (int32_t)grp_xyz.size();
+      me.n_rest = (int64_t)rest.size();
       const size_t rb = A->storage == OAL_STORE_F64 ? 8 : 4;
-      e = cudaMalloc(&me.d_nodes, std::max<size_t>(nodes.size(), 1) * sizeof(int32_t));
-      if (e == cudaSuccess && !nodes.empty()) e = cudaMemcpy(me.d_nodes, nodes.data(), nodes.size() * sizeof(int32_t), cudaMemcpyHostToDevice);
-      if (e == cudaSuccess) e = cudaMalloc(&me.d_node_map, map.size() * sizeof(int32_t));
-      if (e == cudaSuccess) e = cudaMemcpy(me.d_node_map, map.data(), map.size() * sizeof(int32_t), cudaMemcpyHostToDevice);
+      auto put = [&](auto** dst, const auto& src) {
+        if (e != cudaSuccess) return;
+        const size_t bytes = src.size() * sizeof(src[0]);
+        e = cudaMalloc(dst, std::max<size_t>(bytes, 16));
+        if (e == cudaSuccess && bytes) e = cudaMemcpy(*dst, src.data(), bytes, cudaMemcpyHostToDevice);
+      };
+      put(&me.d_nodes, nodes);
+      put(&me.d_node_map, map);
+      put(&me.d_grp_xyz, grp_xyz);
+      put(&me.d_grp_nodes, grp_nodes);
+      put(&me.d_grp_mem, grp_mem);
+      put(&me.d_rest, rest);
       if (e == cudaSuccess) e = cudaMalloc(&me.d_node_vals, std::max<size_t>(nodes.size(), 1) * 32 * rb);
-      me.n_pos = (int32_t)pos_xyz.size();
-      const size_t np1 = std::max<size_t>(pos_xyz.size(), 1);
-      if (e == cudaSuccess) e = cudaMalloc(&me.d_pos_xyz, np1 * sizeof(int4));
-      if (e == cudaSuccess) e = cudaMalloc(&me.d_slot_pos, slot_pos.size() * sizeof(int32_t));
-      if (e == cudaSuccess) e = cudaMalloc(&me.d_pos_nodes, np1 * 64 * sizeof(int32_t));
-      if (e == cudaSuccess) e = cudaMalloc(&me.d_pos_macro, np1 * 4 * rb);
-      if (e == cudaSuccess && me.n_pos > 0) {
-        e = cudaMemcpy(me.d_pos_xyz, pos_xyz.data(), pos_xyz.size() * sizeof(int4), cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = cudaMemcpy(me.d_pos_nodes, pos_nodes.data(), pos_nodes.size() * sizeof(int32_t), cudaMemcpyHostToDevice);
-      }
-      if (e == cudaSuccess) e = cudaMemcpy(me.d_slot_pos, slot_pos.data(), slot_pos.size() * sizeof(int32_t), cudaMemcpyHostToDevice);
-      // a refined level's fill runs in cell-major entry order (block, cell, direction): the
-      // interpolations of one ghost position's directions then read its stencil records together,
-      // which outweighs the coalescing of the direction-major order of plain levels. The order of
-      // entries carries no meaning (each writes its own slot), so the level's geometry is re-ordered
-      // in place.
-      if (e == cudaSuccess && g->n_gentries > 0) {
-        oal_geometry* gm = const_cast<oal_geometry*>(g);
-        auto key = [](const uint2& v) {
-          return ((uint64_t)v.x << 14) | ((uint64_t)(v.y & 511u) << 5) | (uint64_t)((v.y >> 9) & 31u);
-        };
-        std::stable_sort(gm->h_gentries.begin(), gm->h_gentries.end(),
-                         [&](const uint2& p, const uint2& q) { return key(p) < key(q); });
-        e = cudaMemcpy(gm->d_gentries, gm->h_gentries.data(), gm->h_gentries.size() * sizeof(uint2), cudaMemcpyHostToDevice);
-      }
     }
     if (e != cudaSuccess) {
       cudaGetLastError();

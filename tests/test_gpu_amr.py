@@ -198,3 +198,34 @@ def test_channel_bouzidi_on_the_fine_level(env, storage, tol, sphere):
     ora.advance(P, 2)
     compare(H, ora, 2, tol)
     H.close()
+
+
+# refined block sets whose interpolation groups differ in kind: against the domain faces and corners
+# (no cubic range, partial 2 x 2 x 2 groups), re-entrant and diagonal blocks (ghost blocks shared and
+# duplicated), and a third level flush with the edge of the second (absent stencil nodes)
+REGIONS = {
+    "corner": [((0, 0, 0), (8, 8, 8))],
+    "faces": [((0, 0, 8), (16, 32, 16))],
+    "l_shape": [((8, 8, 8), (24, 16, 16)), ((8, 16, 8), (16, 24, 16))],
+    "diagonal": [((8, 8, 8), (16, 16, 16)), ((16, 16, 16), (24, 24, 24))],
+}
+
+
+@pytest.mark.parametrize("region", sorted(REGIONS))
+@pytest.mark.parametrize("flush_third", [False, True])
+@pytest.mark.parametrize("zwall", [0, 1])
+def test_ghost_groups_of_irregular_regions_fp64(env, region, flush_third, zwall):
+    oracle, amr, solver = env
+    coarse = solver.build_box(4, 4, 4)
+    blocks = sorted({b for lo, hi in REGIONS[region] for b in amr.blocks_in_box(coarse, lo, hi)})
+    doms = [coarse, amr.refine(coarse, blocks)]
+    if flush_third:
+        doms.append(amr.refine(doms[1], range(0, doms[1].n_blocks, 3)))
+    u = 0.05
+    rho_fn = lambda X, Y, Z: 1.0 + 0.002 * np.cos(2 * np.pi * X / 32)  # noqa: E731
+    vel_fn = lambda X, Y, Z: np.stack([u + 0.01 * np.sin(2 * np.pi * Y / 32), 0.01 * np.cos(2 * np.pi * Z / 32),  # noqa: E731
+                                       0.01 * np.sin(2 * np.pi * X / 32)])
+    P = params(amr.level_taus(0.53, len(doms)), c_wale=0.2, u_inlet=u, zwall_bc=zwall)
+    H, ora = run_pair(env, doms, P, "f64", 2, rho_fn, vel_fn)
+    compare(H, ora, len(doms), 1e-10)
+    H.close()
