@@ -186,6 +186,8 @@ struct StepArgs {
   int32_t prefetch_ctas;          // x-pair kernel: CTA j also prefetches CTA j + prefetch_ctas's
                                   // populations and velocities into L2 (0 = off; launch tuning)
   int32_t persistent;             // x-pair kernel: resident CTAs walk the units (launch tuning)
+  int32_t strided;                // uniform kernels: population strides from f_bstride / f_kstride
+                                  // (caller-owned arrays) instead of the library's block-major layout
   int32_t pairs_units;            // set by the launcher: units of a persistent launch (0 = one per CTA)
   const int32_t* fast_rec;        // x-pair kernel: per work entry 32 ints (27-entry neighbour row,
                                   // block coordinates + case, block index), in work-list order

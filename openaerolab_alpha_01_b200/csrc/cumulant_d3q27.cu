@@ -745,7 +745,8 @@ __device__ __forceinline__ void store2(S* __restrict__ f, int64_t i0, int64_t i1
 
 // Library-owned block-major layout: block stride 27*512, direction stride 512 (compile time).
 // IDX = uint32_t when the buffer (real + ghost blocks) has fewer than 2^32 elements.
-template <class S, class V, class IDX>
+// STR: run-time population strides (caller-owned arrays).
+template <class S, class V, class IDX, bool STR = false>
 __global__ void __launch_bounds__(128, OAL_FAST_MIN_CTAS) k_cumulant_fast(const StepArgs a, const int32_t* __restrict__ work) {
   constexpr int NL = Lane<V>::N;  // cells per thread
   constexpr int CPB = 4 / NL;     // CTAs per block
@@ -768,7 +769,7 @@ __global__ void __launch_bounds__(128, OAL_FAST_MIN_CTAS) k_cumulant_fast(const 
   T* __restrict__ rho_out = static_cast<T*>(a.rho_out);
   T* __restrict__ vel_out = static_cast<T*>(a.vel_out);
   const T* __restrict__ vel_in = static_cast<const T*>(a.vel_in);
-  constexpr IDX bst = 27 * kCells, kst = kCells;
+  const IDX bst = STR ? (IDX)a.f_bstride : (IDX)(27 * kCells), kst = STR ? (IDX)a.f_kstride : (IDX)kCells;
   const IDX vcs = (IDX)a.v_cstride;
   const int n_real = a.n_blocks;
 
@@ -977,7 +978,8 @@ template <> __device__ __forceinline__ uint32_t pack_dev<float>(F2) { return 0u;
 // stride 256, row (y, z) stride 4 and 32.
 // One unit (a block's OAL_PAIRS_THREADS / 32 z planes) of the x-pair step; `unit` and `n_units`
 // index the launch's units (the CTA's own in the plain form, a walked sequence in the persistent one).
-template <class S, class IDX, bool POS, bool GEN>
+// STR: run-time population strides (even, in elements) instead of that layout: a caller's arrays.
+template <class S, class IDX, bool POS, bool GEN, bool STR>
 __device__ __forceinline__ void pairs_unit(const StepArgs& a, unsigned unit, unsigned n_units, IDX* s_wbase,
                                            int32_t* s_nbr, int32_t* s_tail, CaseParams& s_cp, int32_t& s_pf) {
   constexpr bool DEV = !std::is_same<S, float>::value;  // 16-bit deviation codec
@@ -985,7 +987,8 @@ __device__ __forceinline__ void pairs_unit(const StepArgs& a, unsigned unit, uns
   using W = typename PairWord<S>::W;
   using V = F2;
   using T = float;
-  constexpr IDX wbst = 27 * kCells / 2, wkst = kCells / 2;
+  const IDX wbst = STR ? (IDX)(a.f_bstride / 2) : (IDX)(27 * kCells / 2);
+  const IDX wkst = STR ? (IDX)(a.f_kstride / 2) : (IDX)(kCells / 2);
   const int tid = threadIdx.x;
   // a CTA covers OAL_PAIRS_THREADS / 32 z planes of a block (one warp per plane); the block's
   // neighbour row, coordinates and index come in one coalesced 128-byte record
@@ -1176,8 +1179,8 @@ __device__ __forceinline__ void pairs_unit(const StepArgs& a, unsigned unit, uns
 // POS: some case of the launch uses the positivity limiter (its code is left out otherwise).
 // GEN: some case of the launch relaxes with omega_bulk, omega3 or omega4 other than 1.
 // PERS: the persistent form, resident CTAs walking the launch's units (launch tuning).
-template <class S, class IDX, bool POS, bool GEN, bool PERS>
-__global__ void __launch_bounds__(OAL_PAIRS_THREADS, ((sizeof(S) == 4 || GEN || POS) ? OAL_PAIRS_WARPS_WIDE : OAL_PAIRS_WARPS) * 32 / OAL_PAIRS_THREADS) k_cumulant_pairs(const StepArgs a, const int32_t* __restrict__ work) {
+template <class S, class IDX, bool POS, bool GEN, bool PERS, bool STR = false>
+__global__ void __launch_bounds__(OAL_PAIRS_THREADS, ((sizeof(S) == 4 || GEN || POS || STR) ? OAL_PAIRS_WARPS_WIDE : OAL_PAIRS_WARPS) * 32 / OAL_PAIRS_THREADS) k_cumulant_pairs(const StepArgs a, const int32_t* __restrict__ work) {
   (void)work;
   __shared__ IDX s_wbase[28];  // first word of each neighbour block
   __shared__ int32_t s_nbr[28];
@@ -1188,10 +1191,10 @@ __global__ void __launch_bounds__(OAL_PAIRS_THREADS, ((sizeof(S) == 4 || GEN || 
     const unsigned n_units = (unsigned)a.pairs_units;
     for (unsigned unit = blockIdx.x; unit < n_units; unit += gridDim.x) {
       if (unit != blockIdx.x) __syncthreads();  // the previous unit no longer reads shared memory
-      pairs_unit<S, IDX, POS, GEN>(a, unit, n_units, s_wbase, s_nbr, s_tail, s_cp, s_pf);
+      pairs_unit<S, IDX, POS, GEN, STR>(a, unit, n_units, s_wbase, s_nbr, s_tail, s_cp, s_pf);
     }
   } else {
-    pairs_unit<S, IDX, POS, GEN>(a, blockIdx.x, gridDim.x, s_wbase, s_nbr, s_tail, s_cp, s_pf);
+    pairs_unit<S, IDX, POS, GEN, STR>(a, blockIdx.x, gridDim.x, s_wbase, s_nbr, s_tail, s_cp, s_pf);
   }
 }
 
@@ -1260,6 +1263,7 @@ __global__ void __launch_bounds__(128) k_cumulant_gen(const StepArgs a, const in
     // opposite word are both read without a branch, so that all loads are in flight together ----
     R A[kQ27];
     S raw[kQ27], rawo[kQ27];
+    const bool cut = halfway && (bflags & BF_NEAR_SOLID);  // elsewhere no link is cut: half the loads
 #pragma unroll
     for (int k = 0; k < kQ27; ++k) {
       const int cx = q27_cx(k), cy = q27_cy(k), cz = q27_cz(k);
@@ -1271,7 +1275,7 @@ __global__ void __launch_bounds__(128) k_cumulant_gen(const StepArgs a, const in
       } else {
         raw[k] = fin[(int64_t)(nb >= 0 ? nb : b) * bst + k * kst + ((sx & 7) | ((sy & 7) << 3) | ((sz & 7) << 6))];
       }
-      rawo[k] = halfway ? fin[own + q27_opp(k) * kst] : raw[k];
+      rawo[k] = cut ? fin[own + q27_opp(k) * kst] : raw[k];
     }
 #pragma unroll
     for (int k = 0; k < kQ27; ++k) {
@@ -1773,7 +1777,22 @@ template <class S, class R>
 cudaError_t launch_fast(const StepArgs& a, const int32_t* work, int n_work, cudaStream_t st) {
   if (n_work <= 0) return cudaSuccess;
   // element count of the buffer (real + ghost blocks) decides the index width
-  const bool idx32 = (uint64_t)a.n_total_blocks * 27u * kCells < (1ull << 32);
+  const bool idx32 = (a.strided ? (uint64_t)(a.n_blocks - 1) * (uint64_t)a.f_bstride + 26u * (uint64_t)a.f_kstride + kCells
+                                : (uint64_t)a.n_total_blocks * 27u * kCells) < (1ull << 32);
+  if (a.strided) {
+    if constexpr (sizeof(R) == 8) {
+      if (idx32) k_cumulant_fast<S, double, uint32_t, true><<<(unsigned)n_work * 4u, 128, 0, st>>>(a, work);
+      else k_cumulant_fast<S, double, int64_t, true><<<(unsigned)n_work * 4u, 128, 0, st>>>(a, work);
+    } else {
+      const unsigned units = (unsigned)n_work * (256u / OAL_PAIRS_THREADS);
+      const bool wide = (a.flags_any & (CF_LIMITER_POSITIVITY | CF_GENERAL_RATES)) != 0;
+      if (wide && idx32) k_cumulant_pairs<S, uint32_t, true, true, false, true><<<units, OAL_PAIRS_THREADS, 0, st>>>(a, work);
+      else if (wide) k_cumulant_pairs<S, int64_t, true, true, false, true><<<units, OAL_PAIRS_THREADS, 0, st>>>(a, work);
+      else if (idx32) k_cumulant_pairs<S, uint32_t, false, false, false, true><<<units, OAL_PAIRS_THREADS, 0, st>>>(a, work);
+      else k_cumulant_pairs<S, int64_t, false, false, false, true><<<units, OAL_PAIRS_THREADS, 0, st>>>(a, work);
+    }
+    return cudaGetLastError();
+  }
   if constexpr (sizeof(R) == 8) {
     if (idx32) k_cumulant_fast<S, double, uint32_t><<<(unsigned)n_work * 4u, 128, 0, st>>>(a, work);
     else k_cumulant_fast<S, double, int64_t><<<(unsigned)n_work * 4u, 128, 0, st>>>(a, work);
