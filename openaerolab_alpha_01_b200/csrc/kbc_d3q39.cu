@@ -1820,20 +1820,26 @@ struct KbcLevel {
   int parity = 0;
   int64_t bytes = 0;
   cudaStream_t cap = nullptr;
-  cudaGraphExec_t exec = nullptr;
-  cudaGraph_t graph = nullptr;
-  int32_t g_n = 0;
-  int g_parity = -1;
-  oal_step_params g_p{};
+  // the captured steps by starting parity: an odd number of steps ends on the other buffer
+  struct Graph {
+    cudaGraphExec_t exec = nullptr;
+    cudaGraph_t graph = nullptr;
+    int32_t n = 0;
+    oal_step_params p{};
+  } gr[2];
   bool exact_math = false;  // kbc_set_exact_math
 };
 
 namespace {
 
+void release_graph(KbcLevel::Graph& G) {
+  if (G.exec) cudaGraphExecDestroy(G.exec);
+  if (G.graph) cudaGraphDestroy(G.graph);
+  G = KbcLevel::Graph{};
+}
 void release_graph(KbcLevel* L) {
-  if (L->exec) cudaGraphExecDestroy(L->exec);
-  if (L->graph) cudaGraphDestroy(L->graph);
-  L->exec = nullptr; L->graph = nullptr; L->g_n = 0; L->g_parity = -1;
+  release_graph(L->gr[0]);
+  release_graph(L->gr[1]);
 }
 
 oal_status resolve(const oal_step_params* p, KbcArgs* a) {
@@ -2104,9 +2110,10 @@ oal_status kbc_advance(KbcLevel* L, const oal_step_params* p, int32_t n, void* s
   KBC_TRY(cudaSetDevice(L->device));
   oal_step_params key = *p;
   if (!(p->inlet_turbulence > 0.0f && L->n_entries > 0)) key.time_step_seed = 0;  // the seed only feeds inlet noise
-  const bool hit = L->exec && L->g_n == n && L->g_parity == L->parity && std::memcmp(&L->g_p, &key, sizeof key) == 0;
+  KbcLevel::Graph& G = L->gr[L->parity];
+  const bool hit = G.exec && G.n == n && std::memcmp(&G.p, &key, sizeof key) == 0;
   if (!hit) {
-    release_graph(L);
+    release_graph(G);
     const int start = L->parity;
     KBC_TRY(cudaStreamBeginCapture(L->cap, cudaStreamCaptureModeThreadLocal));
     oal_status es = OAL_OK;
@@ -2123,9 +2130,9 @@ oal_status kbc_advance(KbcLevel* L, const oal_step_params* p, int32_t n, void* s
       cudaGetLastError();
       return fail(OAL_E_CUDA, "graph instantiate: %s", cudaGetErrorString(e));
     }
-    L->exec = exec; L->graph = graph; L->g_n = n; L->g_parity = start; L->g_p = key;
+    G.exec = exec; G.graph = graph; G.n = n; G.p = key;
   }
-  KBC_TRY(cudaGraphLaunch(L->exec, static_cast<cudaStream_t>(stream)));
+  KBC_TRY(cudaGraphLaunch(G.exec, static_cast<cudaStream_t>(stream)));
   if (n & 1) L->parity ^= 1;
   return OAL_OK;
 }
