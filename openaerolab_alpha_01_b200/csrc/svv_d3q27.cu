@@ -19,6 +19,7 @@
 // shared memory (the thread's own column) for the correction. HBM traffic per fluid cell: the
 // 27 input populations once, the 27 output populations read and written.
 #include "svv_d3q27.h"
+#include "vmath.cuh"
 
 namespace oal {
 
@@ -123,29 +124,51 @@ __global__ void __launch_bounds__(svv_threads<R>(), 3) k_svv(const SvvArgs a, co
 // the lane's own input population), so every lane computes exactly what the one-cell kernel does.
 template <class S> struct PairIO;
 template <> struct PairIO<float> {
-  static __device__ __forceinline__ float2 load(const float* p, float, float) { return *reinterpret_cast<const float2*>(p); }
-  static __device__ __forceinline__ void store(float* p, float a, float b, float, float) {
+  static __device__ __forceinline__ F2 load(const float* p, float) {
+    const float2 v = *reinterpret_cast<const float2*>(p);
+    return f2(v.x, v.y);
+  }
+  static __device__ __forceinline__ void store(float* p, F2 v, float) {
+    float a, b;
+    f2split(v, a, b);
     *reinterpret_cast<float2*>(p) = make_float2(a, b);
   }
 };
 template <> struct PairIO<__half> {
-  static __device__ __forceinline__ float2 load(const __half* p, float w, float) {
+  static __device__ __forceinline__ F2 load(const __half* p, float w) {
     const float2 h = __half22float2(*reinterpret_cast<const __half2*>(p));
-    return make_float2(fmaf(w, h.x, w), fmaf(w, h.y, w));
+    return vfma(splat<F2>(w), f2(h.x, h.y), splat<F2>(w));
   }
-  static __device__ __forceinline__ void store(__half* p, float a, float b, float, float inv_w) {
-    *reinterpret_cast<__half2*>(p) = __floats2half2_rn(fmaf(a, inv_w, -1.0f), fmaf(b, inv_w, -1.0f));
+  static __device__ __forceinline__ void store(__half* p, F2 v, float inv_w) {
+    float a, b;
+    f2split(vfma(v, splat<F2>(inv_w), splat<F2>(-1.0f)), a, b);
+    *reinterpret_cast<__half2*>(p) = __floats2half2_rn(a, b);
   }
 };
 template <> struct PairIO<__nv_bfloat16> {
-  static __device__ __forceinline__ float2 load(const __nv_bfloat16* p, float w, float) {
+  static __device__ __forceinline__ F2 load(const __nv_bfloat16* p, float w) {
     const float2 h = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p));
-    return make_float2(fmaf(w, h.x, w), fmaf(w, h.y, w));
+    return vfma(splat<F2>(w), f2(h.x, h.y), splat<F2>(w));
   }
-  static __device__ __forceinline__ void store(__nv_bfloat16* p, float a, float b, float, float inv_w) {
-    *reinterpret_cast<__nv_bfloat162*>(p) = __floats2bfloat162_rn(fmaf(a, inv_w, -1.0f), fmaf(b, inv_w, -1.0f));
+  static __device__ __forceinline__ void store(__nv_bfloat16* p, F2 v, float inv_w) {
+    float a, b;
+    f2split(vfma(v, splat<F2>(inv_w), splat<F2>(-1.0f)), a, b);
+    *reinterpret_cast<__nv_bfloat162*>(p) = __floats2bfloat162_rn(a, b);
   }
 };
+// max(v, 1e-12) per lane that keeps a NaN
+__device__ __forceinline__ float floor_pop(float v) {
+  float r;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(v), "f"(1e-12f));
+  return r;
+}
+// the rounded product c v of both lanes by scalar multiplies: a packed multiply whose result a packed
+// add consumes may be contracted into one packed FMA, a scalar one may not (-fmad=false)
+__device__ __forceinline__ F2 scale2(float c, F2 v) {
+  float a, b;
+  f2split(v, a, b);
+  return f2(c * a, c * b);
+}
 
 // the direction-0 offset of the pair starting at (x, y, z) + d (x + dx even), whether its block
 // exists, and per lane whether the target cell is solid
@@ -163,58 +186,67 @@ __device__ __forceinline__ IDX svv_pair_offset(const SvvArgs& a, int b, int x, i
   const int c = (nx & 7) | ((ny & 7) << 3) | ((nz & 7) << 6);
   s0 = svv_solid(a, bb, c);
   s1 = svv_solid(a, bb, c + 1);
-  return (IDX)a.pi(bb, c, 0);
+  return s0 && s1 ? own : (IDX)a.pi(bb, c, 0);
 }
 
-// the filter of the 27 directions of a pair of cells: the filtered values into s_fl, the changes
-// of mass and momentum of each lane into acc; PICK: some tap of the pair falls back
-template <class S, class IDX, bool PICK>
+// The filter of the 27 directions of a pair of cells, unrolled (weights, velocities and, in the
+// library's layout (KST = 512), the directions' offsets are immediates), in packed f32x2 arithmetic
+// with the oracle's rounding: products with 4 and with +-1 and 0 are exact, so their multiply-adds are
+// one rounding either way; the other products are taken apart (scale2). Filtered values go to s_fl,
+// the changes of mass and momentum to acc. PICK: some tap of the pair falls back in one lane only (a
+// missing block or two solid cells give the pair's own offset instead).
+template <class S, class IDX, bool PICK, int KST>
 __device__ __forceinline__ void svv_pairs_filter(const SvvArgs& a, const S* __restrict__ fin, const S* __restrict__ fout,
-                                                 IDX own, IDX kst, const IDX (&t)[10], uint32_t fb, bool fx, bool fyz,
-                                                 float (*s_fl)[256], int l0, float (&acc)[8]) {
+                                                 IDX own, const IDX (&t)[10], uint32_t fb, bool fx, bool fyz,
+                                                 F2 (*s_fl)[128], F2 (&acc)[4]) {
   const float ex = a.eps_x, eyz = a.eps_yz;
-  float r0 = 0.0f, x0 = 0.0f, y0 = 0.0f, z0 = 0.0f, r1 = 0.0f, x1 = 0.0f, y1 = 0.0f, z1 = 0.0f;
-#pragma unroll 3
+  const IDX kst = KST ? (IDX)KST : (IDX)a.pi.kst;
+  const F2 m4 = splat<F2>(-4.0f);
+#pragma unroll
+  for (int m = 0; m < 4; ++m) acc[m] = splat<F2>(0.0f);
+#pragma unroll
   for (int k = 0; k < kQ27; ++k) {
-    const float w = float(q27_w(k)), inv_w = float(1.0 / q27_w(k));
+    const float w = float(q27_w(k));
     const S* fk = fin + (IDX)k * kst;
-    const float2 o = PairIO<S>::load(fk + own, w, inv_w);  // the pair's own input populations
-    const float2 fc = PairIO<S>::load(fout + own + (IDX)k * kst, w, inv_w);
-    auto pick = [&](int bit, float v, float mine) {
-      if constexpr (PICK) return ((fb >> bit) & 1u) ? mine : v;
+    const F2 o = PairIO<S>::load(fk + own, w);  // the pair's own input populations
+    const F2 fc = PairIO<S>::load(fout + own + (IDX)k * kst, w);
+    const F2 six = scale2(6.0f, fc);
+    // lane 0 takes bit, lane 1 bit + 1 of fb
+    auto pick = [&](int bit, F2 v, F2 mine) {
+      if constexpr (PICK)
+        return f2(((fb >> bit) & 1u) ? f2lo(mine) : f2lo(v), ((fb >> (bit + 1)) & 1u) ? f2hi(mine) : f2hi(v));
       else return v;
     };
-    float bl0 = 0.0f, bl1 = 0.0f;
+    auto lap = [&](F2 t0, F2 t1, F2 t2, F2 t3) { return vfma(m4, t2, vfma(m4, t1, t0) + six) + t3; };
+    F2 bl = splat<F2>(0.0f);
     if (fx) {
-      const float2 m = PairIO<S>::load(fk + t[0], w, inv_w), p = PairIO<S>::load(fk + t[1], w, inv_w);
-      bl0 += ex * ((((pick(0, m.x, o.x) - 4.0f * pick(2, m.y, o.x)) + 6.0f * fc.x) - 4.0f * pick(4, o.y, o.x)) +
-                   pick(6, p.x, o.x));
-      bl1 += ex * ((((pick(1, m.y, o.y) - 4.0f * pick(3, o.x, o.y)) + 6.0f * fc.y) - 4.0f * pick(5, p.x, o.y)) +
-                   pick(7, p.y, o.y));
+      // x - 2, x - 1, x + 1, x + 2 of the two lanes from the pairs (x-2, x-1), (x, x+1), (x+2, x+3)
+      const F2 m = PairIO<S>::load(fk + t[0], w), p = PairIO<S>::load(fk + t[1], w);
+      bl = scale2(ex, lap(pick(0, m, o), pick(2, f2(f2hi(m), f2lo(o)), o), pick(4, f2(f2hi(o), f2lo(p)), o), pick(6, p, o)));
     }
     if (fyz) {
 #pragma unroll
       for (int a2 = 0; a2 < 2; ++a2) {
         const int j0 = 2 + 4 * a2, bit = 8 + 8 * a2;
-        const float2 v0 = PairIO<S>::load(fk + t[j0], w, inv_w), v1 = PairIO<S>::load(fk + t[j0 + 1], w, inv_w);
-        const float2 v2 = PairIO<S>::load(fk + t[j0 + 2], w, inv_w), v3 = PairIO<S>::load(fk + t[j0 + 3], w, inv_w);
-        bl0 += eyz * ((((pick(bit, v0.x, o.x) - 4.0f * pick(bit + 2, v1.x, o.x)) + 6.0f * fc.x) -
-                       4.0f * pick(bit + 4, v2.x, o.x)) + pick(bit + 6, v3.x, o.x));
-        bl1 += eyz * ((((pick(bit + 1, v0.y, o.y) - 4.0f * pick(bit + 3, v1.y, o.y)) + 6.0f * fc.y) -
-                       4.0f * pick(bit + 5, v2.y, o.y)) + pick(bit + 7, v3.y, o.y));
+        const F2 v0 = PairIO<S>::load(fk + t[j0], w), v1 = PairIO<S>::load(fk + t[j0 + 1], w);
+        const F2 v2 = PairIO<S>::load(fk + t[j0 + 2], w), v3 = PairIO<S>::load(fk + t[j0 + 3], w);
+        bl = bl + scale2(eyz, lap(pick(bit, v0, o), pick(bit + 2, v1, o), pick(bit + 4, v2, o), pick(bit + 6, v3, o)));
       }
     }
-    const float f0 = fc.x - bl0, f1 = fc.y - bl1;
-    const float e0 = f0 - fc.x, e1 = f1 - fc.y;
-    r0 += e0; x0 += e0 * float(q27_cx(k)); y0 += e0 * float(q27_cy(k)); z0 += e0 * float(q27_cz(k));
-    r1 += e1; x1 += e1 * float(q27_cx(k)); y1 += e1 * float(q27_cy(k)); z1 += e1 * float(q27_cz(k));
-    s_fl[k][l0] = f0;
-    s_fl[k][l0 + 1] = f1;
+    const F2 f = fc - bl, e = f - fc;
+    acc[0] = acc[0] + e;
+    acc[1] = vfma(e, splat<F2>(float(q27_cx(k))), acc[1]);
+    acc[2] = vfma(e, splat<F2>(float(q27_cy(k))), acc[2]);
+    acc[3] = vfma(e, splat<F2>(float(q27_cz(k))), acc[3]);
+    s_fl[k][threadIdx.x] = f;
   }
-  acc[0] = r0; acc[1] = x0; acc[2] = y0; acc[3] = z0; acc[4] = r1; acc[5] = x1; acc[6] = y1; acc[7] = z1;
 }
 
-template <class S, class IDX>
+// Bound by issue and load latency. The first form of this kernel looped over the directions with the
+// weights, velocities and addresses formed at run time (290 instructions per pair and direction, 651 us
+// for the 256 x 128 x 128 channel in FP16, 620 us in FP32); unrolled and packed it is ~80. The domain
+// faces take the path without selects, because a missing block's taps already point at the pair itself.
+template <class S, class IDX, int KST>
 __global__ void __launch_bounds__(128, 6) k_svv_pairs(const SvvArgs a, const S* __restrict__ fin, S* __restrict__ fout,
                                                       S* __restrict__ fpost2) {
   const int b = blockIdx.x >> 1;
@@ -225,7 +257,7 @@ __global__ void __launch_bounds__(128, 6) k_svv_pairs(const SvvArgs a, const S* 
   const bool d0 = svv_solid(a, b, c0), d1 = svv_solid(a, b, c0 + 1);
   if (d0 && d1) return;
   const IDX own = (IDX)a.pi(b, c0, 0);
-  const IDX kst = (IDX)a.pi.kst;
+  const IDX kst = KST ? (IDX)KST : (IDX)a.pi.kst;
   const bool fx = a.eps_x > 0.0f, fyz = a.eps_yz > 0.0f;
   // pair taps: 0 (x-2, x-1), 1 (x+2, x+3), 2-5 y-2, y-1, y+1, y+2, 6-9 z-2 .. z+2; fb bit 2j + lane:
   // the lane takes its own input population for tap j (x taps: j 0-3 of the lane's x-2 .. x+2)
@@ -244,24 +276,23 @@ __global__ void __launch_bounds__(128, 6) k_svv_pairs(const SvvArgs a, const S* 
     const int s = (j & 3) < 2 ? (j & 3) - 2 : (j & 3) - 1;
     bool q0 = true, q1 = true;
     t[2 + j] = fyz ? svv_pair_offset<IDX>(a, b, x, y, z, 0, j < 4 ? s : 0, j < 4 ? 0 : s, own, q0, q1) : own;
-    fb |= (uint32_t)q0 << (8 + 2 * j) | (uint32_t)q1 << (9 + 2 * j);
+    if (q0 != q1) fb |= (uint32_t)q0 << (8 + 2 * j) | (uint32_t)q1 << (9 + 2 * j);
   }
-  __shared__ float s_fl[kQ27][256];
-  float acc[8];
-  // the fall-back selects only where a tap of the pair falls back (cells next to a solid or a
-  // missing block); elsewhere the loads are used as they are
-  if (fb == 0) svv_pairs_filter<S, IDX, false>(a, fin, fout, own, kst, t, fb, fx, fyz, s_fl, l0, acc);
-  else svv_pairs_filter<S, IDX, true>(a, fin, fout, own, kst, t, fb, fx, fyz, s_fl, l0, acc);
-  const float r0 = acc[0], x0 = acc[1], y0 = acc[2], z0 = acc[3], r1 = acc[4], x1 = acc[5], y1 = acc[6], z1 = acc[7];
+  __shared__ F2 s_fl[kQ27][128];
+  F2 acc[4];
+  // the fall-back selects only where one lane of a tap falls back (cells next to a solid; x taps also
+  // next to a missing block); elsewhere the loads are used as they are
+  if (fb == 0) svv_pairs_filter<S, IDX, false, KST>(a, fin, fout, own, t, fb, fx, fyz, s_fl, acc);
+  else svv_pairs_filter<S, IDX, true, KST>(a, fin, fout, own, t, fb, fx, fyz, s_fl, acc);
   const float inv_cs2 = 1.0f / float(1.0 / 3.0);  // CS2_LATTICE
-#pragma unroll 3
+#pragma unroll
   for (int k = 0; k < kQ27; ++k) {
     const float w = float(q27_w(k)), inv_w = float(1.0 / q27_w(k));
-    const float cx = float(q27_cx(k)), cy = float(q27_cy(k)), cz = float(q27_cz(k));
-    float v0 = s_fl[k][l0] - w * (r0 + inv_cs2 * ((cx * x0 + cy * y0) + cz * z0));
-    float v1 = s_fl[k][l0 + 1] - w * (r1 + inv_cs2 * ((cx * x1 + cy * y1) + cz * z1));
-    v0 = v0 < 1e-12f ? 1e-12f : v0;  // NaN passes
-    v1 = v1 < 1e-12f ? 1e-12f : v1;
+    // (cx jx + cy jy) + cz jz: exact products
+    const F2 cu = vfma(splat<F2>(float(q27_cz(k))), acc[3],
+                       vfma(splat<F2>(float(q27_cy(k))), acc[2], scale2(float(q27_cx(k)), acc[1])));
+    const F2 v = s_fl[k][threadIdx.x] - scale2(w, acc[0] + scale2(inv_cs2, cu));
+    const float v0 = floor_pop(f2lo(v)), v1 = floor_pop(f2hi(v));
     // a solid cell of the pair keeps its stored word
     if (d0 || d1) {
       S* q = fout + own + (IDX)k * kst;
@@ -269,8 +300,8 @@ __global__ void __launch_bounds__(128, 6) k_svv_pairs(const SvvArgs a, const S* 
       if (!d0) { q[0] = Codec<S>::enc(v0, w, inv_w); if (q2) q2[0] = q[0]; }
       if (!d1) { q[1] = Codec<S>::enc(v1, w, inv_w); if (q2) q2[1] = q[1]; }
     } else {
-      PairIO<S>::store(fout + own + (IDX)k * kst, v0, v1, w, inv_w);
-      if (fpost2) PairIO<S>::store(fpost2 + own + (IDX)k * kst, v0, v1, w, inv_w);
+      PairIO<S>::store(fout + own + (IDX)k * kst, f2(v0, v1), inv_w);
+      if (fpost2) PairIO<S>::store(fpost2 + own + (IDX)k * kst, f2(v0, v1), inv_w);
     }
   }
 }
@@ -288,10 +319,12 @@ cudaError_t enqueue_t(const SvvArgs& a, const void* fin, void* fout, void* fpost
     // on a word (every block layout this library allocates; a caller's arrays are checked)
     auto aligned = [](const void* p) { return p == nullptr || ((uintptr_t)p % (2 * sizeof(S))) == 0; };
     if (!a.pi.dense && a.pi.bst % 2 == 0 && a.pi.kst % 2 == 0 && aligned(fin) && aligned(fout) && aligned(fpost2)) {
-      if (n_elements < (int64_t(1) << 32))
-        k_svv_pairs<S, uint32_t><<<(unsigned)nb * 2u, 128, 0, st>>>(a, in, out, post);
-      else
-        k_svv_pairs<S, int64_t><<<(unsigned)nb * 2u, 128, 0, st>>>(a, in, out, post);
+      const bool idx32 = n_elements < (int64_t(1) << 32), own_layout = a.pi.kst == kCells;
+      const unsigned ctas = (unsigned)nb * 2u;
+      if (own_layout && idx32) k_svv_pairs<S, uint32_t, kCells><<<ctas, 128, 0, st>>>(a, in, out, post);
+      else if (own_layout) k_svv_pairs<S, int64_t, kCells><<<ctas, 128, 0, st>>>(a, in, out, post);
+      else if (idx32) k_svv_pairs<S, uint32_t, 0><<<ctas, 128, 0, st>>>(a, in, out, post);
+      else k_svv_pairs<S, int64_t, 0><<<ctas, 128, 0, st>>>(a, in, out, post);
       return cudaGetLastError();
     }
   }
