@@ -313,23 +313,38 @@ struct WallArgs {
   T uin0, uin1, uin2;
 };
 
-// staged neighbour rows of the CTA's octs; returns the number of octs of this CTA
+// Neighbour rows of the warp's four octs, staged in its own part of shared memory; returns the calling
+// lane's oct (8 lanes each), -1 past the end of the work. A warp waits for its own rows only: with one
+// stage per CTA every warp waited for the slowest row of 32 octs before its first pull.
+constexpr int kOctsPerWarp = 4;
 template <class T>
-__device__ __forceinline__ int stage_octs(const LevelArgs<T>& a, int32_t* s_nb, int64_t* s_o) {
-  const int64_t w0 = (int64_t)blockIdx.x * kOctsPerCta;
-  const int64_t total = a.n_work;
-  const int64_t left = total - w0;
-  const int n_here = left < kOctsPerCta ? (int)left : kOctsPerCta;
-  if (threadIdx.x < n_here) s_o[threadIdx.x] = a.work ? (int64_t)a.work[w0 + threadIdx.x] : w0 + threadIdx.x;
-  __syncthreads();
-  for (int t = threadIdx.x; t < n_here * 27; t += kThreads) s_nb[t] = a.onbr[s_o[t / 27] * 27 + t % 27] - 1;
-  __syncthreads();
-  return n_here;
+__device__ __forceinline__ int64_t stage_octs(const LevelArgs<T>& a, int32_t (*s_rows)[27 * kOctsPerWarp]) {
+  const int lane = threadIdx.x & 31;
+  int32_t* rows = s_rows[threadIdx.x >> 5];
+  const int64_t w0 = ((int64_t)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5)) * kOctsPerWarp;
+  const int64_t left = (int64_t)a.n_work - w0;
+  const int n_here = left < kOctsPerWarp ? (left > 0 ? (int)left : 0) : kOctsPerWarp;
+  const int lo = lane >> 3;
+  const int32_t o = lo < n_here ? (a.work ? a.work[w0 + lo] : (int32_t)(w0 + lo)) : -1;
+#pragma unroll
+  for (int j = 0; j < (27 * kOctsPerWarp + 31) / 32; ++j) {
+    const int t = 32 * j + lane, r = t / 27;
+    const int32_t of = __shfl_sync(0xffffffffu, o, (r < kOctsPerWarp ? r : 0) * 8);
+    if (r < n_here) rows[t] = a.onbr[(int64_t)of * 27 + (t - 27 * r)] - 1;
+  }
+  __syncwarp();
+  return o;
+}
+
+// element `index` of array p by a byte offset of type I (32 bits where the array allows it)
+template <class I, class T>
+__device__ __forceinline__ T load_at(const T* p, I index) {
+  return __ldg(reinterpret_cast<const T*>(reinterpret_cast<const char*>(p) + (I)(index * (I)sizeof(T))));
 }
 
 // central differences of the previous step's velocity over the 6 face neighbours (stream.jl:13-30);
 // WALLS: a missing or domain-boundary neighbour contributes the slot's own velocity
-template <class T, bool WALLS>
+template <class T, bool WALLS, class I>
 __device__ __forceinline__ void velocity_gradient(const LevelArgs<T>& a, const uint8_t* kind, const int32_t* nb, int64_t o,
                                                   int k, T* g) {
   const int x = k & 1, y = (k >> 1) & 1, z = (k >> 2) & 1;
@@ -341,15 +356,15 @@ __device__ __forceinline__ void velocity_gradient(const LevelArgs<T>& a, const u
       const int d = s == 0 ? 1 : -1;
       const int nx = x + (ax == 0 ? d : 0), ny = y + (ax == 1 ? d : 0), nz = z + (ax == 2 ? d : 0);
       const int ox = nx < 0 ? -1 : (nx > 1 ? 1 : 0), oy = ny < 0 ? -1 : (ny > 1 ? 1 : 0), oz = nz < 0 ? -1 : (nz > 1 ? 1 : 0);
-      int64_t no = nb[nbr_slot_index(ox, oy, oz)];
+      I no = (I)nb[nbr_slot_index(ox, oy, oz)];
       int nk = (nx - 2 * ox) + 2 * (ny - 2 * oy) + 4 * (nz - 2 * oz);
-      if (WALLS && (no < 0 || kind[no * 8 + nk] == K_BOUNDARY)) {
-        no = o;
+      if (WALLS && (nb[nbr_slot_index(ox, oy, oz)] < 0 || kind[(int64_t)no * 8 + nk] == K_BOUNDARY)) {
+        no = (I)o;
         nk = k;
       }
       T* v = s == 0 ? vp : vm;
 #pragma unroll
-      for (int c = 0; c < 3; ++c) v[c] = __ldg(a.uin + no * 24 + 8 * c + nk);
+      for (int c = 0; c < 3; ++c) v[c] = load_at<I>(a.uin, no * (I)24 + (I)(8 * c + nk));
     }
     const T h = T(0.5);
 #pragma unroll
@@ -358,14 +373,14 @@ __device__ __forceinline__ void velocity_gradient(const LevelArgs<T>& a, const u
 }
 
 // subgrid viscosity, omega and the HRR stress of slot (k, o) (stream.jl:357-360)
-template <class T, int SGS, bool GRAD, bool WALLS>
+template <class T, int SGS, bool GRAD, bool WALLS, class I = int64_t>
 __device__ __forceinline__ T relaxation(const LevelArgs<T>& a, const uint8_t* kind, const int32_t* nb, int64_t o, int k,
                                         T* pfd) {
 #pragma unroll
   for (int n = 0; n < 6; ++n) pfd[n] = T(0);
   if (!GRAD) return a.omega0;
   T g[9];
-  velocity_gradient<T, WALLS>(a, kind, nb, o, k, g);
+  velocity_gradient<T, WALLS, I>(a, kind, nb, o, k, g);
   T nut = T(0);
   if (SGS == 1) nut = nu_wale<T>(g, a.cw);
   if (SGS == 2) nut = nu_smagorinsky<T>(g, a.cs);
@@ -399,15 +414,17 @@ __device__ __forceinline__ void store_cell(const LevelArgs<T>& a, int64_t o, int
 
 // octs whose eight slots are plain fluid cells (every pull source is a fluid slot)
 // SGS: 0 none, 1 WALE, 2 Smagorinsky, 3 Vreman; GRAD: the velocity gradient is needed (SGS or HRR)
-template <class T, int SGS, bool GRAD, bool FORCED>
+// I: the type of byte offsets into the level's arrays (32 bits below 4 GB: a multiply-add per pull
+// instead of a 64-bit chain). Bound by the latency of the gathers and by issue (no multiply-add may be
+// fused). 192^3 periodic FP32 level, WALE + HRR, two steps: 880 us with 64-bit offsets and rows staged
+// per CTA, 747 us now (3.5 TB/s of its algorithmic bytes).
+template <class T, int SGS, bool GRAD, bool FORCED, class I>
 __global__ void __launch_bounds__(kThreads) k_q19_step(const LevelArgs<T> a) {
-  __shared__ int32_t s_nb[kOctsPerCta * 27];
-  __shared__ int64_t s_o[kOctsPerCta];
-  const int n_here = stage_octs<T>(a, s_nb, s_o);
-  const int lo = threadIdx.x >> 3, k = threadIdx.x & 7;
-  if (lo >= n_here) return;
-  const int64_t o = s_o[lo];
-  const int32_t* nb = s_nb + 27 * lo;
+  __shared__ int32_t s_rows[kThreads / 32][27 * kOctsPerWarp];
+  const int64_t o = stage_octs<T>(a, s_rows);
+  if (o < 0) return;
+  const int k = threadIdx.x & 7;
+  const int32_t* nb = s_rows[threadIdx.x >> 5] + 27 * ((threadIdx.x >> 3) & 3);
   const int x = k & 1, y = (k >> 1) & 1, z = (k >> 2) & 1;
 
   // pull: slot k takes direction i from slot (x,y,z) - c_i, in this oct or a neighbour (octree.jl:139-150)
@@ -415,13 +432,12 @@ __global__ void __launch_bounds__(kThreads) k_q19_step(const LevelArgs<T> a) {
 #pragma unroll
   for (int i = 0; i < Q; ++i) {
     const int px = x - cx(i), py = y - cy(i), pz = z - cz(i);
-    const int ox = px < 0 ? -1 : (px > 1 ? 1 : 0), oy = py < 0 ? -1 : (py > 1 ? 1 : 0), oz = pz < 0 ? -1 : (pz > 1 ? 1 : 0);
-    const int src = nb[nbr_slot_index(ox, oy, oz)];
-    const int child = (px - 2 * ox) + 2 * (py - 2 * oy) + 4 * (pz - 2 * oz);
-    f[i] = __ldg(a.fin + (int64_t)src * (8 * Q) + 8 * i + child);
+    // (p >> 1) is -1, 0 or 1: the neighbour oct; p & 1 the child there
+    const I src = (I)nb[(px >> 1) + 3 * (py >> 1) + 9 * (pz >> 1) + 13];
+    f[i] = load_at<I>(a.fin, src * (I)(8 * Q) + (I)(8 * i + ((px & 1) | ((py & 1) << 1) | ((pz & 1) << 2))));
   }
   T pfd[6];
-  const T omega = relaxation<T, SGS, GRAD, false>(a, nullptr, nb, o, k, pfd);
+  const T omega = relaxation<T, SGS, GRAD, false, I>(a, nullptr, nb, o, k, pfd);
   T out[Q], rho, ux, uy, uz;
   collide<T>(f, omega, a.sigma, pfd, a.F0, a.F1, a.F2, FORCED, out, rho, ux, uy, uz);
   store_cell<T>(a, o, k, out, rho, ux, uy, uz);
@@ -483,15 +499,13 @@ __device__ __forceinline__ T face_population(const WallArgs<T>& w, uint32_t mask
 // Bouzidi rule on cut links and the momentum exchange (stream.jl:205-257)
 template <class T, int SGS, bool GRAD, bool FORCED>
 __global__ void __launch_bounds__(kThreads) k_q19_walls(const LevelArgs<T> a, const WallArgs<T> w) {
-  __shared__ int32_t s_nb[kOctsPerCta * 27];
-  __shared__ int64_t s_o[kOctsPerCta];
-  const int n_here = stage_octs<T>(a, s_nb, s_o);
-  const int lo = threadIdx.x >> 3, k = threadIdx.x & 7;
-  if (lo >= n_here) return;
-  const int64_t o = s_o[lo];
+  __shared__ int32_t s_rows[kThreads / 32][27 * kOctsPerWarp];
+  const int64_t o = stage_octs<T>(a, s_rows);
+  if (o < 0) return;
+  const int k = threadIdx.x & 7;
   const int64_t s = o * 8 + k;
   if (w.kind[s] != K_FLUID) return;
-  const int32_t* nb = s_nb + 27 * lo;
+  const int32_t* nb = s_rows[threadIdx.x >> 5] + 27 * ((threadIdx.x >> 3) & 3);
   const int x = k & 1, y = (k >> 1) & 1, z = (k >> 2) & 1;
   const uint32_t sp = w.special[s];
   T f[Q];
@@ -864,8 +878,11 @@ cudaError_t launch3(const LevelArgs<T>& a, const WallArgs<T>* w, bool forced, cu
   const int64_t n = a.n_work;
   if (n > 0) {
     const unsigned grid = (unsigned)((n + kOctsPerCta - 1) / kOctsPerCta);
-    if (forced) k_q19_step<T, SGS, GRAD, true><<<grid, kThreads, 0, st>>>(a);
-    else k_q19_step<T, SGS, GRAD, false><<<grid, kThreads, 0, st>>>(a);
+    const bool small = (uint64_t)a.nocts * (8 * Q * sizeof(T)) < (uint64_t(1) << 32);
+    if (forced && small) k_q19_step<T, SGS, GRAD, true, uint32_t><<<grid, kThreads, 0, st>>>(a);
+    else if (forced) k_q19_step<T, SGS, GRAD, true, int64_t><<<grid, kThreads, 0, st>>>(a);
+    else if (small) k_q19_step<T, SGS, GRAD, false, uint32_t><<<grid, kThreads, 0, st>>>(a);
+    else k_q19_step<T, SGS, GRAD, false, int64_t><<<grid, kThreads, 0, st>>>(a);
   }
   (void)w;
   return cudaGetLastError();
@@ -1536,13 +1553,29 @@ __global__ void __launch_bounds__(256) k_q19_fill(int32_t ng, const int32_t* __r
   const unsigned gmask = 0xffffu << (lane & 16);
   T acc = T(0);
   if (q < 10) {
-    const int32_t* dx = dix + 64 * g;
-    const float* w = gw + 64 * g;
-#pragma unroll 8
-    for (int n = 0; n < 64; ++n) {
-      const int32_t d = __ldg(dx + n);
-      if (!d) continue;
-      acc += T(__ldg(w + n)) * __ldg(dm + 10 * (int64_t)(d - 1) + q);
+    // the 64 nodes in node order, their reads 32 at a time: the kernel is a few warps per SM waiting on
+    // index -> moment reads, two trips per batch (8 at a time: sixteen trips)
+    const int4* dx = reinterpret_cast<const int4*>(dix + 64 * g);
+    const float4* w = reinterpret_cast<const float4*>(gw + 64 * g);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      int32_t d[32];
+      T v[32];
+#pragma unroll
+      for (int n = 0; n < 8; ++n) {
+        const int4 t = __ldg(dx + 8 * h + n);
+        d[4 * n] = t.x; d[4 * n + 1] = t.y; d[4 * n + 2] = t.z; d[4 * n + 3] = t.w;
+      }
+#pragma unroll
+      for (int n = 0; n < 32; ++n) v[n] = d[n] ? __ldg(dm + 10 * (int64_t)(d[n] - 1) + q) : T(0);
+#pragma unroll
+      for (int n = 0; n < 8; ++n) {
+        const float4 t = __ldg(w + 8 * h + n);
+        const float wn[4] = {t.x, t.y, t.z, t.w};
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+          if (d[4 * n + c]) acc += T(wn[c]) * v[4 * n + c];
+      }
     }
   }
   T m[10];
@@ -1583,10 +1616,21 @@ __global__ void __launch_bounds__(256) k_q19_restrict(int32_t nr, const int32_t*
   int cnt = 0;
   if (cubic[r]) {
     if (q < 10) {
-#pragma unroll 8
-      for (int n = 0; n < 64; ++n) {
-        const T wn = T(restrict_w1(n & 3) * restrict_w1((n >> 2) & 3) * restrict_w1(n >> 4));
-        acc += wn * __ldg(rm + 10 * (int64_t)(__ldg(sx + n) - 1) + q);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        T v[32];
+#pragma unroll
+        for (int n = 0; n < 8; ++n) {
+          const int4 t = __ldg(reinterpret_cast<const int4*>(sx) + 8 * h + n);
+          const int32_t d[4] = {t.x, t.y, t.z, t.w};
+#pragma unroll
+          for (int c = 0; c < 4; ++c) v[4 * n + c] = __ldg(rm + 10 * (int64_t)(d[c] - 1) + q);
+        }
+#pragma unroll
+        for (int n = 0; n < 32; ++n) {
+          const int m = 32 * h + n;
+          acc += T(restrict_w1(m & 3) * restrict_w1((m >> 2) & 3) * restrict_w1(m >> 4)) * v[n];
+        }
       }
     }
   } else {
