@@ -397,7 +397,7 @@ __device__ __forceinline__ R parent_scale(const ParentView& P) {
 // for the macros: 290 + 124 us per substep of the two-level sphere channel (256 x 128 x 128, refined
 // box 96 x 64 x 64, FP16; 131,000 ghost cells).
 template <class S, class R>
-__global__ void __launch_bounds__(128) k_parent_fill(const ParentView P, S* __restrict__ f, int32_t n_real, bool comp) {
+__global__ void __launch_bounds__(128, sizeof(R) == 8 ? 2 : 4) k_parent_fill(const ParentView P, S* __restrict__ f, int32_t n_real, bool comp) {
   const int32_t g = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (g >= P.n_groups) return;
   const int4 gx = P.grp_xyz[g];
@@ -436,30 +436,31 @@ __global__ void __launch_bounds__(128) k_parent_fill(const ParentView P, S* __re
     }
     if (an >= 0) anchor = vals[(int64_t)an * 32];
   }
+  // the 64 ids in two loads a lane, then every record read of the group in flight at once: a warp
+  // waits for two trips to memory (per-quad index loads and 16 records at a time: eight, 112 us)
+  const int32_t id0 = nodes[lane], id1 = nodes[lane + 32];
+  const uint2 mem = lane < 8 ? P.grp_mem[(int64_t)g * 8 + lane] : make_uint2(0u, 0u);
+  R v[4][4][4];
+#pragma unroll
+  for (int i = 0; i < 64; ++i) {
+    const int a = i >> 4, b = (i >> 2) & 3, c = i & 3;
+    const int32_t id = __shfl_sync(0xffffffffu, i < 32 ? id0 : id1, i & 31);
+    // outside the cubic range only the bracket's corners count
+    const bool outer = a == 0 || a == 3 || b == 0 || b == 3 || c == 0 || c == 3;
+    if (outer && !cubic) v[a][b][c] = R(0);
+    else v[a][b][c] = (all || id >= 0) ? vals[(int64_t)id * 32] : anchor;
+  }
   R acc[2][2][2] = {};
 #pragma unroll
   for (int a = 0; a < 4; ++a) {
     R yz[2][2] = {};
-    R v[4][4];
-#pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      const int4 q = reinterpret_cast<const int4*>(nodes)[4 * a + b];
-      const int32_t id[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        // outside the cubic range only the bracket's corners count
-        const bool outer = a == 0 || a == 3 || b == 0 || b == 3 || c == 0 || c == 3;
-        if (outer && !cubic) v[b][c] = R(0);
-        else v[b][c] = (all || id[c] >= 0) ? vals[(int64_t)id[c] * 32] : anchor;
-      }
-    }
 #pragma unroll
     for (int b = 0; b < 4; ++b)
 #pragma unroll
       for (int s = 0; s < 2; ++s) {
-        R z = L[2][s][0] * v[b][0];
+        R z = L[2][s][0] * v[a][b][0];
 #pragma unroll
-        for (int c = 1; c < 4; ++c) z = vfma(L[2][s][c], v[b][c], z);
+        for (int c = 1; c < 4; ++c) z = vfma(L[2][s][c], v[a][b][c], z);
         yz[0][s] = vfma(L[1][0][b], z, yz[0][s]);
         yz[1][s] = vfma(L[1][1][b], z, yz[1][s]);
       }
@@ -477,11 +478,11 @@ __global__ void __launch_bounds__(128) k_parent_fill(const ParentView P, S* __re
   const R iwk = d2 == 0 ? R(27.0 / 8.0) : d2 == 1 ? R(13.5) : d2 == 2 ? R(54) : R(216);
   const R scale = parent_scale<R>(P);
   R own[4] = {R(1), R(0), R(0), R(0)};
-  if (!(cubic && all) && lane < 8 && P.grp_mem[(int64_t)g * 8 + lane].y != 0u)
+  if (!(cubic && all) && mem.y != 0u)
     node_macros<R>(static_cast<const R*>(P.node_vals), P.dim_x * kBS, P.dim_y * kBS, P.dim_z * kBS, nodes, 2 * gx.x + (lane & 1), 2 * gx.y + ((lane >> 1) & 1), 2 * gx.z + (lane >> 2), own);
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
-    const uint2 m = P.grp_mem[(int64_t)g * 8 + j];
+    const uint2 m = make_uint2(__shfl_sync(0xffffffffu, mem.x, j), __shfl_sync(0xffffffffu, mem.y, j));
     if (m.y == 0u) continue;
     const R v = acc[j & 1][(j >> 1) & 1][j >> 2];
     R mac[4];
@@ -1654,11 +1655,12 @@ __global__ void __launch_bounds__(128) k_restrict(const RestrictArgs r) {
   const int lx = (cell & 7) + 1, ly = ((cell >> 3) & 7) + 1, lz = (cell >> 6) + 1;
   const int4 bi = r.pbinfo[pb];
   const int cbx0 = 2 * bi.x - 1, cby0 = 2 * bi.y - 1, cbz0 = 2 * bi.z - 1;
-  int32_t cblk[8], ccell[8];
+  // the children in pairs along x (2 lx - 1, 2 lx: one block, adjacent words)
+  int32_t cblk[4], ccell[4];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int sx = i >> 2, sy = (i >> 1) & 1, sz = i & 1;  // sx outer, sz inner (the reference's order)
-    const int fx = 2 * (lx - 1) + 1 + sx, fy = 2 * (ly - 1) + 1 + sy, fz = 2 * (lz - 1) + 1 + sz;
+  for (int i = 0; i < 4; ++i) {
+    const int sy = i >> 1, sz = i & 1;
+    const int fx = 2 * (lx - 1) + 1, fy = 2 * (ly - 1) + 1 + sy, fz = 2 * (lz - 1) + 1 + sz;
     const int cbx = cbx0 + (fx - 1) / kBS, cby = cby0 + (fy - 1) / kBS, cbz = cbz0 + (fz - 1) / kBS;
     if (cbx < 1 || cby < 1 || cbz < 1 || cbx > r.cdx || cby > r.cdy || cbz > r.cdz) return;
     const int32_t cb = r.cptr[(cbx - 1) + (int64_t)r.cdx * ((cby - 1) + (int64_t)r.cdy * (cbz - 1))];
@@ -1666,19 +1668,30 @@ __global__ void __launch_bounds__(128) k_restrict(const RestrictArgs r) {
     cblk[i] = cb - 1;
     ccell[i] = ((fx - 1) % kBS) | (((fy - 1) % kBS) << 3) | (((fz - 1) % kBS) << 6);
   }
+  struct alignas(2 * sizeof(S)) Pair { S a, b; };
   const S* cf = static_cast<const S*>(r.cf);
   R avg[kQ27];
 #pragma unroll
   for (int k = 0; k < kQ27; ++k) avg[k] = R(0);
   int fluid = 0;
 #pragma unroll 1
-  for (int i = 0; i < 8; ++i) {
+  for (int i = 0; i < 4; ++i) {
     const int cb = cblk[i];
-    if ((r.cbflags[cb] & BF_NEAR_SOLID) && ((r.ccmask[(int64_t)r.cmslot[cb] * kCells + ccell[i]] >> 13) & 1u)) continue;
-    ++fluid;
-    const int64_t base = (int64_t)cb * (27 * kCells) + ccell[i];
+    bool f0 = true, f1 = true;
+    if (r.cbflags[cb] & BF_NEAR_SOLID) {
+      const uint32_t* m = r.ccmask + (int64_t)r.cmslot[cb] * kCells + ccell[i];
+      f0 = !((m[0] >> 13) & 1u);
+      f1 = !((m[1] >> 13) & 1u);
+    }
+    fluid += (int)f0 + (int)f1;
+    const Pair* c = reinterpret_cast<const Pair*>(cf + (int64_t)cb * (27 * kCells) + ccell[i]);
 #pragma unroll
-    for (int k = 0; k < kQ27; ++k) avg[k] += Codec<S>::dec(cf[base + k * kCells], R(q27_w(k)), R(1.0 / q27_w(k)));
+    for (int k = 0; k < kQ27; ++k) {
+      const Pair p = c[k * (kCells / 2)];
+      const R va = Codec<S>::dec(p.a, R(q27_w(k)), R(1.0 / q27_w(k))), vb = Codec<S>::dec(p.b, R(q27_w(k)), R(1.0 / q27_w(k)));
+      avg[k] += f0 ? va : R(0);
+      avg[k] += f1 ? vb : R(0);
+    }
   }
   if (fluid == 0) return;
   const R inv_children = R(1) / R(fluid);
