@@ -18,6 +18,8 @@
 // tap (the block's rows, mostly L1 hits) and the arithmetic. The filtered populations wait in
 // shared memory (the thread's own column) for the correction. HBM traffic per fluid cell: the
 // 27 input populations once, the 27 output populations read and written.
+#include <type_traits>
+
 #include "svv_d3q27.h"
 #include "vmath.cuh"
 
@@ -122,12 +124,17 @@ __global__ void __launch_bounds__(svv_threads<R>(), 3) k_svv(const SvvArgs a, co
 // are adjacent words, and the x taps of the pair come from the pairs (x-2, x-1), (x, x+1) and
 // (x+2, x+3). Each lane keeps its own fall-back flags (a solid target or a missing block selects
 // the lane's own input population), so every lane computes exactly what the one-cell kernel does.
+// W: the pair's stored word, read where the program reads it (a volatile load: the reads ahead of the
+// filter below must not sink to their uses); dec: its two populations (f = w + w d for 16-bit deviations).
 template <class S> struct PairIO;
 template <> struct PairIO<float> {
-  static __device__ __forceinline__ F2 load(const float* p, float) {
-    const float2 v = *reinterpret_cast<const float2*>(p);
-    return f2(v.x, v.y);
+  using W = uint2;
+  static __device__ __forceinline__ W word(const float* p) {
+    W v;
+    asm volatile("ld.global.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+    return v;
   }
+  static __device__ __forceinline__ F2 dec(W v, float) { return f2(__uint_as_float(v.x), __uint_as_float(v.y)); }
   static __device__ __forceinline__ void store(float* p, F2 v, float) {
     float a, b;
     f2split(v, a, b);
@@ -135,8 +142,14 @@ template <> struct PairIO<float> {
   }
 };
 template <> struct PairIO<__half> {
-  static __device__ __forceinline__ F2 load(const __half* p, float w) {
-    const float2 h = __half22float2(*reinterpret_cast<const __half2*>(p));
+  using W = uint32_t;
+  static __device__ __forceinline__ W word(const __half* p) {
+    W v;
+    asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+  }
+  static __device__ __forceinline__ F2 dec(W v, float w) {
+    const float2 h = __half22float2(*reinterpret_cast<const __half2*>(&v));
     return vfma(splat<F2>(w), f2(h.x, h.y), splat<F2>(w));
   }
   static __device__ __forceinline__ void store(__half* p, F2 v, float inv_w) {
@@ -146,8 +159,14 @@ template <> struct PairIO<__half> {
   }
 };
 template <> struct PairIO<__nv_bfloat16> {
-  static __device__ __forceinline__ F2 load(const __nv_bfloat16* p, float w) {
-    const float2 h = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p));
+  using W = uint32_t;
+  static __device__ __forceinline__ W word(const __nv_bfloat16* p) {
+    W v;
+    asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+  }
+  static __device__ __forceinline__ F2 dec(W v, float w) {
+    const float2 h = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v));
     return vfma(splat<F2>(w), f2(h.x, h.y), splat<F2>(w));
   }
   static __device__ __forceinline__ void store(__nv_bfloat16* p, F2 v, float inv_w) {
@@ -195,21 +214,41 @@ __device__ __forceinline__ IDX svv_pair_offset(const SvvArgs& a, int b, int x, i
 // one rounding either way; the other products are taken apart (scale2). Filtered values go to s_fl,
 // the changes of mass and momentum to acc. PICK: some tap of the pair falls back in one lane only (a
 // missing block or two solid cells give the pair's own offset instead).
-template <class S, class IDX, bool PICK, int KST>
+template <class S, class IDX, bool PICK, int KST, bool X>
 __device__ __forceinline__ void svv_pairs_filter(const SvvArgs& a, const S* __restrict__ fin, const S* __restrict__ fout,
-                                                 IDX own, const IDX (&t)[10], uint32_t fb, bool fx, bool fyz,
+                                                 IDX own, const IDX (&t)[10], uint32_t fb, bool fx, bool fyz_x,
                                                  F2 (*s_fl)[128], F2 (&acc)[4]) {
   const float ex = a.eps_x, eyz = a.eps_yz;
   const IDX kst = KST ? (IDX)KST : (IDX)a.pi.kst;
+  const bool fyz = !X || fyz_x;  // X = false: y and z taps only, no branch in the loop
+  using IO = PairIO<S>;
+  using W = typename IO::W;
   const F2 m4 = splat<F2>(-4.0f);
 #pragma unroll
   for (int m = 0; m < 4; ++m) acc[m] = splat<F2>(0.0f);
+  // the words of a direction: own input, own output, the eight y and z taps, the two x pairs; those of
+  // the next directions are on their way while one is filtered (one direction at a time the warps
+  // spent two thirds of their time waiting for its ten reads)
+  constexpr int kAhead = KST == 0 ? 0 : sizeof(S) == 2 ? 2 : 1;  // what the registers hold
+  W q[kAhead + 1][12];
+  auto fetch = [&](int k, W (&d)[12]) {
+    const S* fk = fin + (IDX)k * kst;
+    d[0] = IO::word(fk + own);
+    d[1] = IO::word(fout + own + (IDX)k * kst);
+    if (fyz)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) d[2 + j] = IO::word(fk + t[2 + j]);
+    if (X && fx) { d[10] = IO::word(fk + t[0]); d[11] = IO::word(fk + t[1]); }
+  };
+#pragma unroll
+  for (int k = 0; k < kAhead; ++k) fetch(k, q[k]);  // none where kAhead is 0
 #pragma unroll
   for (int k = 0; k < kQ27; ++k) {
     const float w = float(q27_w(k));
-    const S* fk = fin + (IDX)k * kst;
-    const F2 o = PairIO<S>::load(fk + own, w);  // the pair's own input populations
-    const F2 fc = PairIO<S>::load(fout + own + (IDX)k * kst, w);
+    if (k + kAhead < kQ27) fetch(k + kAhead, q[(k + kAhead) % (kAhead + 1)]);
+    const W (&d)[12] = q[k % (kAhead + 1)];
+    const F2 o = IO::dec(d[0], w);  // the pair's own input populations
+    const F2 fc = IO::dec(d[1], w);
     const F2 six = scale2(6.0f, fc);
     // lane 0 takes bit, lane 1 bit + 1 of fb
     auto pick = [&](int bit, F2 v, F2 mine) {
@@ -219,18 +258,17 @@ __device__ __forceinline__ void svv_pairs_filter(const SvvArgs& a, const S* __re
     };
     auto lap = [&](F2 t0, F2 t1, F2 t2, F2 t3) { return vfma(m4, t2, vfma(m4, t1, t0) + six) + t3; };
     F2 bl = splat<F2>(0.0f);
-    if (fx) {
+    if (X && fx) {
       // x - 2, x - 1, x + 1, x + 2 of the two lanes from the pairs (x-2, x-1), (x, x+1), (x+2, x+3)
-      const F2 m = PairIO<S>::load(fk + t[0], w), p = PairIO<S>::load(fk + t[1], w);
+      const F2 m = IO::dec(d[10], w), p = IO::dec(d[11], w);
       bl = scale2(ex, lap(pick(0, m, o), pick(2, f2(f2hi(m), f2lo(o)), o), pick(4, f2(f2hi(o), f2lo(p)), o), pick(6, p, o)));
     }
     if (fyz) {
 #pragma unroll
       for (int a2 = 0; a2 < 2; ++a2) {
         const int j0 = 2 + 4 * a2, bit = 8 + 8 * a2;
-        const F2 v0 = PairIO<S>::load(fk + t[j0], w), v1 = PairIO<S>::load(fk + t[j0 + 1], w);
-        const F2 v2 = PairIO<S>::load(fk + t[j0 + 2], w), v3 = PairIO<S>::load(fk + t[j0 + 3], w);
-        bl = bl + scale2(eyz, lap(pick(bit, v0, o), pick(bit + 2, v1, o), pick(bit + 4, v2, o), pick(bit + 6, v3, o)));
+        bl = bl + scale2(eyz, lap(pick(bit, IO::dec(d[j0], w), o), pick(bit + 2, IO::dec(d[j0 + 1], w), o),
+                                  pick(bit + 4, IO::dec(d[j0 + 2], w), o), pick(bit + 6, IO::dec(d[j0 + 3], w), o)));
       }
     }
     const F2 f = fc - bl, e = f - fc;
@@ -242,12 +280,15 @@ __device__ __forceinline__ void svv_pairs_filter(const SvvArgs& a, const S* __re
   }
 }
 
-// Bound by issue and load latency. The first form of this kernel looped over the directions with the
-// weights, velocities and addresses formed at run time (290 instructions per pair and direction, 651 us
-// for the 256 x 128 x 128 channel in FP16, 620 us in FP32); unrolled and packed it is ~80. The domain
-// faces take the path without selects, because a missing block's taps already point at the pair itself.
-template <class S, class IDX, int KST>
-__global__ void __launch_bounds__(128, 6) k_svv_pairs(const SvvArgs a, const S* __restrict__ fin, S* __restrict__ fout,
+// Bound by the latency of its DRAM reads: a direction's own input and output words come from DRAM, so
+// the bandwidth follows from the directions a warp has in flight. On the 256 x 128 x 128 channel in
+// FP16, y-z taps: 651 us with the directions in a loop that formed weights, velocities and addresses at
+// run time (290 instructions per pair and direction), 515 us unrolled and packed (~80), 365 us with two
+// directions read ahead at 20 warps per SM. The domain faces take the path without selects, because a
+// missing block's taps already point at the pair itself.
+// X: the x filter is on (then both axes' switches are run-time).
+template <class S, class IDX, int KST, bool X>
+__global__ void __launch_bounds__(128, sizeof(S) == 4 ? 4 : 5) k_svv_pairs(const SvvArgs a, const S* __restrict__ fin, S* __restrict__ fout,
                                                       S* __restrict__ fpost2) {
   const int b = blockIdx.x >> 1;
   const int base = (blockIdx.x & 1) << 8;
@@ -258,7 +299,7 @@ __global__ void __launch_bounds__(128, 6) k_svv_pairs(const SvvArgs a, const S* 
   if (d0 && d1) return;
   const IDX own = (IDX)a.pi(b, c0, 0);
   const IDX kst = KST ? (IDX)KST : (IDX)a.pi.kst;
-  const bool fx = a.eps_x > 0.0f, fyz = a.eps_yz > 0.0f;
+  const bool fx = X && a.eps_x > 0.0f, fyz = !X || a.eps_yz > 0.0f;
   // pair taps: 0 (x-2, x-1), 1 (x+2, x+3), 2-5 y-2, y-1, y+1, y+2, 6-9 z-2 .. z+2; fb bit 2j + lane:
   // the lane takes its own input population for tap j (x taps: j 0-3 of the lane's x-2 .. x+2)
   IDX t[10];
@@ -282,8 +323,8 @@ __global__ void __launch_bounds__(128, 6) k_svv_pairs(const SvvArgs a, const S* 
   F2 acc[4];
   // the fall-back selects only where one lane of a tap falls back (cells next to a solid; x taps also
   // next to a missing block); elsewhere the loads are used as they are
-  if (fb == 0) svv_pairs_filter<S, IDX, false, KST>(a, fin, fout, own, t, fb, fx, fyz, s_fl, acc);
-  else svv_pairs_filter<S, IDX, true, KST>(a, fin, fout, own, t, fb, fx, fyz, s_fl, acc);
+  if (fb == 0) svv_pairs_filter<S, IDX, false, KST, X>(a, fin, fout, own, t, fb, fx, fyz, s_fl, acc);
+  else svv_pairs_filter<S, IDX, true, KST, X>(a, fin, fout, own, t, fb, fx, fyz, s_fl, acc);
   const float inv_cs2 = 1.0f / float(1.0 / 3.0);  // CS2_LATTICE
 #pragma unroll
   for (int k = 0; k < kQ27; ++k) {
@@ -321,10 +362,15 @@ cudaError_t enqueue_t(const SvvArgs& a, const void* fin, void* fout, void* fpost
     if (!a.pi.dense && a.pi.bst % 2 == 0 && a.pi.kst % 2 == 0 && aligned(fin) && aligned(fout) && aligned(fpost2)) {
       const bool idx32 = n_elements < (int64_t(1) << 32), own_layout = a.pi.kst == kCells;
       const unsigned ctas = (unsigned)nb * 2u;
-      if (own_layout && idx32) k_svv_pairs<S, uint32_t, kCells><<<ctas, 128, 0, st>>>(a, in, out, post);
-      else if (own_layout) k_svv_pairs<S, int64_t, kCells><<<ctas, 128, 0, st>>>(a, in, out, post);
-      else if (idx32) k_svv_pairs<S, uint32_t, 0><<<ctas, 128, 0, st>>>(a, in, out, post);
-      else k_svv_pairs<S, int64_t, 0><<<ctas, 128, 0, st>>>(a, in, out, post);
+      auto go = [&](auto x_on) {
+        constexpr bool X = decltype(x_on)::value;
+        if (own_layout && idx32) k_svv_pairs<S, uint32_t, kCells, X><<<ctas, 128, 0, st>>>(a, in, out, post);
+        else if (own_layout) k_svv_pairs<S, int64_t, kCells, X><<<ctas, 128, 0, st>>>(a, in, out, post);
+        else if (idx32) k_svv_pairs<S, uint32_t, 0, X><<<ctas, 128, 0, st>>>(a, in, out, post);
+        else k_svv_pairs<S, int64_t, 0, X><<<ctas, 128, 0, st>>>(a, in, out, post);
+      };
+      if (a.eps_x > 0.0f) go(std::true_type{});
+      else go(std::false_type{});
       return cudaGetLastError();
     }
   }
