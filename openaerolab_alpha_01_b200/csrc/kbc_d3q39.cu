@@ -1081,12 +1081,13 @@ __device__ __forceinline__ void svv_axis(const SvvView a, const Tables& T, const
 // three Newton passes of ~600 and one or two Cholesky solves of ~650, alpha ~1,200, the rest pull,
 // WALE and update) at 168 registers, three CTAs per SM, issue 51 % active (no_instruction and wait
 // stalls: the body is straight-line code). The body is unrolled over the pairs with the 39
-// equilibrium values in registers; the rare paths (guards, clamps, HRR, the other alpha solvers)
-// read the shared columns. Measured on a 96^3 periodic box, two steps per call: 2,660 us with the
+// equilibrium values in registers, guards and blends included; HRR, the other alpha solvers and what
+// follows a NaN read the shared columns. Measured on a 96^3 periodic box, two steps per call: 2,660 us with the
 // Newton pass over the basis table, alpha from sums of logarithms over the columns and a trip to
-// memory per pulled direction; 451 us now while alpha comes from the series, 1,040 us (3,370 before)
+// memory per pulled direction; 452 us now while alpha comes from the series, 722 us (3,370 before)
 // on a developed flow whose deviations are of the order of f_eq, so that every alpha comes from the
-// logarithms. Distance from the 64-bit step after two steps: velocity 3.1e-5 against 2.9e-3 before.
+// logarithms and many cells take the positivity blends, which read the equilibrium from registers
+// and the column (1,040 us while they evaluated it again). Distance from the 64-bit step after two steps: velocity 3.1e-5 against 2.9e-3 before.
 // SVV: the spectral vanishing viscosity is compiled in (a.svv_x or a.svv_yz > 0).
 template <bool EDGES, bool FAST, bool SVV = false>
 __global__ void __launch_bounds__(kThreads, FAST ? KBC_FAST_MIN_BLOCKS : KBC_MIN_BLOCKS) k_kbc_step(const KbcArgs a) {
@@ -1412,17 +1413,31 @@ __global__ void __launch_bounds__(kThreads, FAST ? KBC_FAST_MIN_BLOCKS : KBC_MIN
     if (any_negative) {
       unbalanced = true;
       float worst = 1.0f;
+      if constexpr (FAST) {
+#pragma unroll
+        for (int k = 0; k < Q; ++k) {
+          const float fk = fe[k] * eq.corr, fneq = sf[k * kThreads] - fk;
+          if (fneq < 0.0f && fk > F_FLOOR) worst = jmin(worst, (fk - F_FLOOR) / (-fneq + F_FLOOR));
+        }
+        worst = jclamp(worst, 0.0f, 1.0f);
+#pragma unroll
+        for (int k = 0; k < Q; ++k) {
+          const float fk = fe[k] * eq.corr;
+          sf[k * kThreads] = maxc(fk + worst * (sf[k * kThreads] - fk), F_FLOOR);
+        }
+      } else {
 #pragma unroll 1
-      for (int k = 0; k < Q; ++k) {
-        const float fe = eq(T, k);
-        const float fneq = sf[k * kThreads] - fe;
-        if (fneq < 0.0f && fe > F_FLOOR) worst = jmin(worst, (fe - F_FLOOR) / (-fneq + F_FLOOR));
-      }
-      worst = jclamp(worst, 0.0f, 1.0f);
+        for (int k = 0; k < Q; ++k) {
+          const float fe = eq(T, k);
+          const float fneq = sf[k * kThreads] - fe;
+          if (fneq < 0.0f && fe > F_FLOOR) worst = jmin(worst, (fe - F_FLOOR) / (-fneq + F_FLOOR));
+        }
+        worst = jclamp(worst, 0.0f, 1.0f);
 #pragma unroll 1
-      for (int k = 0; k < Q; ++k) {
-        const float fe = eq(T, k);
-        sf[k * kThreads] = maxc(fe + worst * (sf[k * kThreads] - fe), F_FLOOR);
+        for (int k = 0; k < Q; ++k) {
+          const float fe = eq(T, k);
+          sf[k * kThreads] = maxc(fe + worst * (sf[k * kThreads] - fe), F_FLOOR);
+        }
       }
     }
   }
@@ -1444,25 +1459,43 @@ __global__ void __launch_bounds__(kThreads, FAST ? KBC_FAST_MIN_BLOCKS : KBC_MIN
     if (eq_limited || macro_limited) guard = jmax(guard, 1.0f);
     if (guard > 0.0f) {
       float sdf = 0.0f, sfe = 0.0f;
+      if constexpr (FAST) {
+#pragma unroll
+        for (int k = 0; k < Q; ++k) {
+          const float fk = fe[k] * eq.corr;
+          sdf += fabsf(sf[k * kThreads] - fk);
+          sfe += fk;
+        }
+      } else {
 #pragma unroll 1
-      for (int k = 0; k < Q; ++k) {
-        const float fe = eq(T, k);
-        sdf += fabsf(sf[k * kThreads] - fe);
-        sfe += fabsf(fe);
+        for (int k = 0; k < Q; ++k) {
+          const float fe = eq(T, k);
+          sdf += fabsf(sf[k * kThreads] - fe);
+          sfe += fabsf(fe);
+        }
       }
       const float reps = sfe > 1e-10f ? sdf / sfe : 0.0f;
       const float cap = jmax(0.025f, 0.18f - 0.155f * guard);
       if (reps > cap) {
         const float th = jclamp(cap / jmax(reps, 1e-12f), 0.0f, 1.0f);
+        if constexpr (FAST) {
+#pragma unroll
+          for (int k = 0; k < Q; ++k) {
+            const float fk = fe[k] * eq.corr;
+            sf[k * kThreads] = maxc(fk + th * (sf[k * kThreads] - fk), F_FLOOR);
+          }
+        } else {
 #pragma unroll 1
-        for (int k = 0; k < Q; ++k) {
-          const float fe = eq(T, k);
-          sf[k * kThreads] = maxc(fe + th * (sf[k * kThreads] - fe), F_FLOOR);
+          for (int k = 0; k < Q; ++k) {
+            const float fe = eq(T, k);
+            sf[k * kThreads] = maxc(fe + th * (sf[k * kThreads] - fe), F_FLOOR);
+          }
         }
       }
     }
   }
-  bool post_done = false;  // the fast path's column holds the post-collision populations
+  bool post_done = false;  // the fast path's column holds the post-collision populations ...
+  bool blended = false;    // ... after the positivity blend and the guard
   if constexpr (FAST) {
     if (a.solver == 0 && !hr.on) {
       const float coeff_s = 1.0f - 2.0f * beta;
@@ -1480,12 +1513,17 @@ __global__ void __launch_bounds__(kThreads, FAST ? KBC_FAST_MIN_BLOCKS : KBC_MIN
       // the arriving populations
       float hv[19], h_sq = 0.0f;
       {
+        // f_eq takes the column's place, for the post-collision blends
         float H0 = entropy_term(sf[0], 0, 0.0f), H1 = 0.0f;
-        fe[0] = fe[0] + coeff_s * (sf[0] - fe[0]);
+        const float f0 = sf[0];
+        sf[0] = fe[0];
+        fe[0] = fe[0] + coeff_s * (f0 - fe[0]);
 #pragma unroll
         for (int p = 0; p < 19; ++p) {
           const int k = kpos(p), kb = kopp(k);
           const float fk = sf[k * kThreads], fb = sf[kb * kThreads];
+          sf[k * kThreads] = fe[k];
+          sf[kb * kThreads] = fe[kb];
           if (!decided) {
             H0 = entropy_term(fk, k, H0);
             H1 = entropy_term(fb, kb, H1);
@@ -1508,7 +1546,7 @@ __global__ void __launch_bounds__(kThreads, FAST ? KBC_FAST_MIN_BLOCKS : KBC_MIN
           }
         }
       }
-      // KBC update; every population and their sum checked before the store
+      // KBC update; the smallest population and their sum checked before the store
       const float coeff = 1.0f - 2.0f * beta * alpha_f;
       float low = fe[0], total = fe[0];
 #pragma unroll
@@ -1519,12 +1557,51 @@ __global__ void __launch_bounds__(kThreads, FAST ? KBC_FAST_MIN_BLOCKS : KBC_MIN
         low = fminf(low, fminf(fe[k], fe[kb]));
         total += fe[k] + fe[kb];
       }
-      if (!SVV && !(guard > 0.0f) && low >= 0.0f && total <= 1e3f) {  // nothing below zero, above 1e3 or NaN
+      const bool sane = total <= 1e3f;  // no population above 1e3 beside the negative ones, no NaN
+      if (sane && low < 0.0f) {
+        // positivity blend toward f_eq (as in the general tail)
+        float blend = 1.0f;
+#pragma unroll
+        for (int k = 0; k < Q; ++k) {
+          const float fk = sf[k * kThreads], fneq = fe[k] - fk;
+          if (fneq < 0.0f && fk > F_FLOOR) blend = fminf(blend, fk / (fk - fneq + F_FLOOR));
+        }
+        blend = fmaxf(blend, 0.0f);
+#pragma unroll
+        for (int k = 0; k < Q; ++k) {
+          const float fk = sf[k * kThreads];
+          fe[k] = fk + blend * (fe[k] - fk);
+        }
+      }
+      if (sane && guard > 0.0f) {
+        float sdf = 0.0f, sfe = 0.0f;
+#pragma unroll
+        for (int k = 0; k < Q; ++k) {
+          const float fk = sf[k * kThreads];
+          sdf += fabsf(fe[k] - fk);
+          sfe += fk;
+        }
+        const float ep = sfe > 1e-10f ? sdf / sfe : 0.0f;
+        const float cap = fmaxf(0.025f, 0.22f - 0.195f * guard);
+        if (ep > cap) {
+          const float th = jclamp(cap / fmaxf(ep, 1e-12f), 0.0f, 1.0f);
+#pragma unroll
+          for (int k = 0; k < Q; ++k) {
+            const float fk = sf[k * kThreads];
+            fe[k] = maxc(fk + th * (fe[k] - fk), F_FLOOR);
+          }
+        }
+      }
+      float top = fe[0];
+#pragma unroll
+      for (int k = 1; k < Q; ++k) top = fmaxf(top, fe[k]);
+      if (!SVV && sane && top <= 1e3f) {
         float* fo = a.fout + (int64_t)b * Q * 512 + cell;
 #pragma unroll
         for (int k = 0; k < Q; ++k) fo[k * 512] = fe[k];
         return;
       }
+      blended = sane;
 #pragma unroll
       for (int k = 0; k < Q; ++k) sf[k * kThreads] = fe[k];
       post_done = true;
@@ -1598,7 +1675,7 @@ __global__ void __launch_bounds__(kThreads, FAST ? KBC_FAST_MIN_BLOCKS : KBC_MIN
       fmin = jmin(fmin, v);
     }
   }
-  if (fmin < 0.0f) {
+  if (fmin < 0.0f && !blended) {
     float blend = 1.0f;
 #pragma unroll 1
     for (int k = 0; k < Q; ++k) {
@@ -1613,7 +1690,7 @@ __global__ void __launch_bounds__(kThreads, FAST ? KBC_FAST_MIN_BLOCKS : KBC_MIN
       sf[k * kThreads] = fe + blend * (sf[k * kThreads] - fe);
     }
   }
-  if (guard > 0.0f) {
+  if (guard > 0.0f && !blended) {
     float sdf = 0.0f, sfe = 0.0f;
 #pragma unroll 1
     for (int k = 0; k < Q; ++k) {
