@@ -112,8 +112,9 @@ struct ParentView {
   const void* vel_old;
   const int32_t* ptr;   // [dim_x*dim_y*dim_z], x fastest: 1-based parent block, 0 = none
   int32_t dim_x, dim_y, dim_z, nb;
-  double tau_parent, tau_fine, tw;
-  int32_t use_temporal, level_visc_physical;
+  double tw;
+  double scale;         // rescaling of the interpolated f_neq (physics_interpolation.jl:1131-1198)
+  int32_t use_temporal;
   // parent nodes evaluated once per substep (k_parent_nodes): node_map[parent cell] = record index
   // or -1; record = 32 values of the compute type: blended rho, ux, uy, uz, then f_neq of the 27
   // directions. Null: evaluate nodes on the fly.

@@ -374,19 +374,6 @@ __device__ __noinline__ void node_macros(const R* vals, int pnx, int pny, int pn
   out[0] = rho_i; out[1] = ux_i; out[2] = uy_i; out[3] = uz_i;
 }
 
-// the rescaling of the interpolated f_neq (:1131-1198)
-template <class R>
-__device__ __forceinline__ R parent_scale(const ParentView& P) {
-  const R tau_p = R(P.tau_parent), tau_f = R(P.tau_fine);
-  const R tau_c = tau_p - R(0.5), tau_fm = tau_f - R(0.5);
-  R scale = tau_c > R(1e-6) ? fmin(fmax(tau_fm / tau_c, R(0.01)), R(100)) : R(1);
-  if (P.level_visc_physical == 1) scale = fmin(fmax(tau_f / (R(2) * fmax(tau_p, R(0.500001))), R(0.01)), R(100));
-  const R omega_c = R(1) / fmax(tau_p, R(0.500001)), omega_f = R(1) / fmax(tau_f, R(0.500001));
-  const R one_m_wc = R(1) - omega_c, one_m_wf = R(1) - omega_f;
-  if (fabs(one_m_wc) > R(1e-6)) scale = fmin(fmax(scale * (one_m_wf / one_m_wc), R(0.01)), R(100));
-  return scale;
-}
-
 // One warp per group of 2 x 2 x 2 fine cells that share their parent bracket (p + 1/4 and p + 3/4 per
 // axis) and so their 64-node stencil. Lane l carries value l of every record (rho, u, the f_neq of the
 // 27 directions), so a node is one coalesced 128-byte read, read once for all eight cells and all
@@ -404,26 +391,20 @@ __global__ void __launch_bounds__(128, sizeof(R) == 8 ? 2 : 4) k_parent_fill(con
   const int32_t* nodes = P.grp_nodes + (int64_t)g * 64;
   const R* __restrict__ vals = static_cast<const R*>(P.node_vals) + lane;
   const bool cubic = (gx.w & GF_CUBIC) != 0, all = (gx.w & GF_ALL_NODES) != 0;
-  // per axis and parity of the fine coordinate: the weights of the four nodes
+  // per axis and parity of the fine coordinate the weights of the four nodes, one per lane (24), then
+  // shared out: every lane evaluating all 24 was a third of the kernel's instructions
   R L[3][2][4];
-#pragma unroll
-  for (int ax = 0; ax < 3; ++ax) {
+  {
+    const int ax = lane >> 3 < 3 ? lane >> 3 : 2, sp = (lane >> 2) & 1, i = lane & 3;
     const int h = ax == 0 ? gx.x : ax == 1 ? gx.y : gx.z;
     const int n = (ax == 0 ? P.dim_x : ax == 1 ? P.dim_y : P.dim_z) * kBS;
+    int i0, i1;
+    R w;
+    parent_bracket<R>(R(2 * h + sp) * R(0.5) + R(0.25), n, i0, i1, w);
+    // trilinear between the bracket's corners outside the cubic range
+    const R l = cubic ? lagrange3<R>(i - 1, w) : (i == 1 ? R(1) - w : i == 2 ? w : R(0));
 #pragma unroll
-    for (int s = 0; s < 2; ++s) {
-      int i0, i1;
-      R w;
-      parent_bracket<R>(R(2 * h + s) * R(0.5) + R(0.25), n, i0, i1, w);
-      if (cubic) {
-        const Lagrange4<R> l(w);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) L[ax][s][i] = l.v[i];
-      } else {
-        // trilinear between the bracket's corners
-        L[ax][s][0] = R(0); L[ax][s][1] = R(1) - w; L[ax][s][2] = w; L[ax][s][3] = R(0);
-      }
-    }
+    for (int m = 0; m < 24; ++m) L[m >> 3][(m >> 2) & 1][m & 3] = __shfl_sync(0xffffffffu, l, m);
   }
   // an absent node counts as the first existing corner (order 000, 100, 010, 110, 001, ...), or 0
   R anchor = R(0);
@@ -476,7 +457,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 8 ? 2 : 4) k_parent_fill(con
   const int cxi = k % 3 - 1, cyi = (k / 3) % 3 - 1, czi = k / 9 - 1, d2 = cxi * cxi + cyi * cyi + czi * czi;
   const R wk = d2 == 0 ? R(8.0 / 27.0) : d2 == 1 ? R(2.0 / 27.0) : d2 == 2 ? R(1.0 / 54.0) : R(1.0 / 216.0);
   const R iwk = d2 == 0 ? R(27.0 / 8.0) : d2 == 1 ? R(13.5) : d2 == 2 ? R(54) : R(216);
-  const R scale = parent_scale<R>(P);
+  const R scale = R(P.scale);
   R own[4] = {R(1), R(0), R(0), R(0)};
   if (!(cubic && all) && mem.y != 0u)
     node_macros<R>(static_cast<const R*>(P.node_vals), P.dim_x * kBS, P.dim_y * kBS, P.dim_z * kBS, nodes, 2 * gx.x + (lane & 1), 2 * gx.y + ((lane >> 1) & 1), 2 * gx.z + (lane >> 2), own);
@@ -576,7 +557,7 @@ __device__ __noinline__ R parent_population(const ParentView& P, int fgx, int fg
   } else {
     f_neq = trilin(&PNode<R>::fneq);
   }
-  return feq_i + f_neq * parent_scale<R>(P);
+  return feq_i + f_neq * R(P.scale);
 }
 
 // Population arriving at cell (x,y,z) of block b in direction k from outside every block

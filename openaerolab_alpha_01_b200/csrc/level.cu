@@ -2253,6 +2253,21 @@ static double restrict_ratio(R tau_p, R tau_c, int physical) {
   return (double)r;
 }
 
+// The rescaling of the f_neq interpolated from the parent, (tau_f - 1/2) / (tau_c - 1/2) or the
+// physical rule, times the post-collision factor (physics_interpolation.jl:1131-1198), in the level's
+// arithmetic.
+template <class R>
+static double parent_scale(float tau_parent, float tau_fine, int physical) {
+  const R tau_p = R(tau_parent), tau_f = R(tau_fine);
+  const R tau_c = tau_p - R(0.5), tau_fm = tau_f - R(0.5);
+  R scale = tau_c > R(1e-6) ? std::fmin(std::fmax(tau_fm / tau_c, R(0.01)), R(100)) : R(1);
+  if (physical == 1) scale = std::fmin(std::fmax(tau_f / (R(2) * std::fmax(tau_p, R(0.500001))), R(0.01)), R(100));
+  const R omega_c = R(1) / std::fmax(tau_p, R(0.500001)), omega_f = R(1) / std::fmax(tau_f, R(0.500001));
+  const R one_m_wc = R(1) - omega_c, one_m_wf = R(1) - omega_f;
+  if (std::fabs(one_m_wc) > R(1e-6)) scale = std::fmin(std::fmax(scale * (one_m_wf / one_m_wc), R(0.01)), R(100));
+  return (double)scale;
+}
+
 // One step of level l (0-based) and, recursively, two substeps of each finer level, then the
 // restriction onto l. t_sub: the level's step index (noise seed); tw: temporal weight of l's parent.
 static oal_status amr_step(oal_amr* A, int l, const std::vector<CaseParams>& cps, const oal_step_params* P,
@@ -2284,11 +2299,10 @@ static oal_status amr_step(oal_amr* A, int l, const std::vector<CaseParams>& cps
     v.ptr = pa.d_ptr;
     v.dim_x = pa.dim[0]; v.dim_y = pa.dim[1]; v.dim_z = pa.dim[2];
     v.nb = pa.g->nb;
-    v.tau_parent = P[l - 1].tau;
-    v.tau_fine = P[l].tau;
+    v.scale = A->storage == OAL_STORE_F64 ? parent_scale<double>(P[l - 1].tau, P[l].tau, P[l].level_visc_physical)
+                                          : parent_scale<float>(P[l - 1].tau, P[l].tau, P[l].level_visc_physical);
     v.tw = tw;
     v.use_temporal = 1;  // TEMPORAL_INTERPOLATION (config_loader.jl:90)
-    v.level_visc_physical = P[l].level_visc_physical;
     v.node_map = me.d_node_map;
     v.node_vals = me.d_node_vals;
     v.nodes = me.d_nodes;
