@@ -187,6 +187,7 @@ struct StepArgs {
   int32_t prefetch_ctas;          // x-pair kernel: CTA j also prefetches CTA j + prefetch_ctas's
                                   // populations and velocities into L2 (0 = off; launch tuning)
   int32_t persistent;             // x-pair kernel: resident CTAs walk the units (launch tuning)
+  int32_t faces;                  // caller-owned arrays: a missing neighbour (-1) is a domain face
   int32_t strided;                // uniform kernels: population strides from f_bstride / f_kstride
                                   // (caller-owned arrays) instead of the library's block-major layout
   int32_t pairs_units;            // set by the launcher: units of a persistent launch (0 = one per CTA)

@@ -636,15 +636,6 @@ __device__ __forceinline__ R face_population_impl(const S* __restrict__ fin, int
   return vfma(R(1) - beta, v, beta * fe);
 }
 
-// The general kernel calls the face logic from 27 unrolled sites; one out-of-line copy keeps
-// its code small.
-template <class S, class R>
-__device__ __noinline__ R face_population(const S* __restrict__ fin, int64_t bbase, int cell, int64_t kst,
-                                           const int32_t* nbr, int n_real, int64_t bst, int k, int x, int y, int z,
-                                           int gx, int gy, int gz, const CaseParams& cp) {
-  return face_population_impl<S, R>(fin, bbase, cell, kst, nbr, n_real, bst, k, x, y, z, gx, gy, gz, cp);
-}
-
 __device__ __forceinline__ const CaseParams& case_of(const StepArgs& a, int case_id) {
   return a.cases ? a.cases[case_id] : a.p0;
 }
@@ -1183,20 +1174,32 @@ __global__ void __launch_bounds__(OAL_PAIRS_THREADS, ((sizeof(S) == 4 || GEN || 
 // ------------------------------------------------------------------------------------------------
 // general kernel: one cell per thread, every option
 // ------------------------------------------------------------------------------------------------
-template <class S, class R, bool DENSE>
-__global__ void __launch_bounds__(128) k_cumulant_gen(const StepArgs a, const int32_t* __restrict__ work) {
+// FACES: pulls may leave the blocks (caller-owned arrays); levels have ghost blocks there, and their
+// instance carries none of that code (within one instance its registers cost the sphere channel 1 %
+// and the two-level one 3 %).
+template <class S, class R, bool DENSE, bool FACES>
+__global__ void __launch_bounds__(128, FACES && sizeof(R) == 4 ? 4 : 3) k_cumulant_gen(const StepArgs a, const int32_t* __restrict__ work) {
   __shared__ int32_t s_nbr[28];
+  __shared__ int64_t s_base[28];  // first element of each neighbour block (the block's own where missing)
   __shared__ CaseParams s_cp;
   __shared__ double s_mom[4][3];
+  // caller-owned arrays: the populations that cross a domain face, one column per thread
+  __shared__ R s_face[FACES ? kQ27 : 1][FACES ? 128 : 1];
   const int tid = threadIdx.x;
   const int b = work ? work[blockIdx.x >> 2] : a.block_base + (int)(blockIdx.x >> 2);
   const int part = blockIdx.x & 3;
-  if (tid < 27) s_nbr[tid] = a.nbr[(int64_t)b * 27 + tid];
+  if (tid < 27) {
+    const int32_t v = a.nbr[(int64_t)b * 27 + tid];
+    s_nbr[tid] = v;
+    s_base[tid] = (int64_t)(v >= 0 ? v : b) * a.f_bstride;
+  }
   const int4 bi = a.binfo[b];
   if (tid >= 32 && tid < 32 + (int)(sizeof(CaseParams) / 4))
     reinterpret_cast<uint32_t*>(&s_cp)[tid - 32] =
         reinterpret_cast<const uint32_t*>(&case_of(a, a.cases ? bi.w : 0))[tid - 32];
-  __syncthreads();
+  bool missing = false;
+  if constexpr (FACES) missing = __syncthreads_or(tid < 27 && s_nbr[tid] < 0) != 0;
+  else __syncthreads();
   const CaseParams& cp = s_cp;
   const uint32_t flags = cp.flags;
   const uint32_t bflags = a.bflags[b];
@@ -1243,6 +1246,30 @@ __global__ void __launch_bounds__(128) k_cumulant_gen(const StepArgs a, const in
     // ---- pull (kernel_cumulant.jl:190-400): where every source lies in a block (ghost blocks
     // included), the stored word of the neighbour and, for half-way links, the own cell's
     // opposite word are both read without a branch, so that all loads are in flight together ----
+    // pulls that leave the caller's blocks (no ghost blocks there): bit k of `miss`. At the default
+    // boundary options a face value is the inlet equilibrium or one of the cell's own populations of
+    // the same weight (outlet, mirrors), so the pull only changes its address; the other options go
+    // through the full face logic in a rolled loop (27 unrolled call sites of it kept 168 registers
+    // and made the kernel wait for instructions: 145 us for the 1,288 face and sphere blocks of a
+    // 192 x 96 x 96 channel in FP32)
+    uint32_t miss = 0;
+    const bool plain_faces = !(flags & (CF_ZWALL_SLIP | CF_ZWALL_NOSLIP | CF_TRANSVERSE_FS | CF_YMIN_WALL));
+    if (FACES && missing) {
+#pragma unroll
+      for (int k = 0; k < kQ27; ++k) {
+        const int sx = x - q27_cx(k), sy = y - q27_cy(k), sz = z - q27_cz(k);
+        miss |= s_nbr[nbr_dir(sx >> 3, sy >> 3, sz >> 3)] < 0 ? 1u << k : 0u;
+      }
+      if (!plain_faces) {
+#pragma unroll 1
+        for (int k = 0; k < kQ27; ++k)
+          if ((miss >> k) & 1u)
+            s_face[FACES ? k : 0][FACES ? tid : 0] = face_population_impl<S, R>(fin, (int64_t)b * bst, cell, kst, s_nbr, n_real, bst, k, x, y, z, gx, gy, gz, cp);
+      }
+    }
+    // the cell's position at the domain faces
+    const bool x_lo = gx == 1, x_hi = gx == cp.nx, y_lo = gy == 1, y_hi = gy == cp.ny, z_lo = gz == 1, z_hi = gz == cp.nz;
+    const R u_inst = R(cp.u_inlet) + R((flags & CF_INLET_NOISE) ? gradient_noise(gy, gz, cp.time_step_seed, 1234) * cp.inlet_turbulence * cp.u_inlet : 0.0f);
     R A[kQ27];
     S raw[kQ27], rawo[kQ27];
     const bool cut = halfway && (bflags & BF_NEAR_SOLID);  // elsewhere no link is cut: half the loads
@@ -1250,22 +1277,25 @@ __global__ void __launch_bounds__(128) k_cumulant_gen(const StepArgs a, const in
     for (int k = 0; k < kQ27; ++k) {
       const int cx = q27_cx(k), cy = q27_cy(k), cz = q27_cz(k);
       const int sx = x - cx, sy = y - cy, sz = z - cz;
-      const int nb = DENSE ? 0 : s_nbr[nbr_dir(sx >> 3, sy >> 3, sz >> 3)];
       if (DENSE) {
         // the padded grid holds every source, ghost frame included
         raw[k] = fin[own - cx - (int64_t)cy * a.PX - (int64_t)cz * a.PX * a.PY + k * kst];
       } else {
-        raw[k] = fin[(int64_t)(nb >= 0 ? nb : b) * bst + k * kst + ((sx & 7) | ((sy & 7) << 3) | ((sz & 7) << 6))];
+        int64_t e = s_base[nbr_dir(sx >> 3, sy >> 3, sz >> 3)] + ((sx & 7) | ((sy & 7) << 3) | ((sz & 7) << 6)) + k * kst;
+        if (FACES && missing && ((miss >> k) & 1u)) {
+          // own cell: direction k beyond the outlet, its mirror beyond y, else beyond z
+          const bool out = cx < 0 && x_hi, yo = (cy > 0 && y_lo) || (cy < 0 && y_hi);
+          e = own + (out ? k : yo ? q27_mir_y(k) : q27_mir_z(k)) * kst;
+        }
+        raw[k] = fin[e];
       }
       rawo[k] = cut ? fin[own + q27_opp(k) * kst] : raw[k];
     }
 #pragma unroll
     for (int k = 0; k < kQ27; ++k) {
       const int cx = q27_cx(k), cy = q27_cy(k), cz = q27_cz(k);
-      const int sx = x - cx, sy = y - cy, sz = z - cz;
-      const int nb = DENSE ? 0 : s_nbr[nbr_dir(sx >> 3, sy >> 3, sz >> 3)];
       R val;
-      if (DENSE || nb >= 0) {
+      if (!FACES || !missing || !((miss >> k) & 1u)) {
         if (halfway && ((mask >> k) & 1u)) {
           // the link opp(k) of this cell is cut: its own post-collision population returns
           const int i = q27_opp(k);
@@ -1279,7 +1309,15 @@ __global__ void __launch_bounds__(128) k_cumulant_gen(const StepArgs a, const in
           val = Codec<S>::dec(raw[k], R(q27_w(k)), R(1.0 / q27_w(k)));
         }
       } else {
-        val = face_population<S, R>(fin, (int64_t)b * bst, cell, kst, s_nbr, n_real, bst, k, x, y, z, gx, gy, gz, cp);
+        if (!plain_faces) {
+          val = s_face[FACES ? k : 0][FACES ? tid : 0];
+        } else if (cx > 0 && x_lo) {
+          val = feq_k<R>(k, R(1), u_inst, R(0), R(0), (flags & CF_COMPRESSIBLE) != 0);
+        } else {
+          // a copy, or a block missing inside the domain (kernel_cumulant.jl:389-391)
+          const bool face = (cx < 0 && x_hi) || (cy > 0 && y_lo) || (cy < 0 && y_hi) || (cz > 0 && z_lo) || (cz < 0 && z_hi);
+          val = face ? Codec<S>::dec(raw[k], R(q27_w(k)), R(1.0 / q27_w(k))) : R(q27_w(k));
+        }
       }
       A[k] = val;
     }
@@ -1771,8 +1809,11 @@ template <class S, class R>
 cudaError_t launch_fast(const StepArgs& a, const int32_t* work, int n_work, cudaStream_t st) {
   if (n_work <= 0) return cudaSuccess;
   // element count of the buffer (real + ghost blocks) decides the index width
-  const bool idx32 = (a.strided ? (uint64_t)(a.n_blocks - 1) * (uint64_t)a.f_bstride + 26u * (uint64_t)a.f_kstride + kCells
-                                : (uint64_t)a.n_total_blocks * 27u * kCells) < (1ull << 32);
+  // (a caller's velocity stride counts too)
+  const uint64_t most = a.strided ? std::max((uint64_t)(a.n_blocks - 1) * (uint64_t)a.f_bstride + 26u * (uint64_t)a.f_kstride + kCells,
+                                             2u * (uint64_t)a.v_cstride + (uint64_t)a.n_blocks * kCells)
+                                  : (uint64_t)a.n_total_blocks * 27u * kCells;
+  const bool idx32 = most < (1ull << 32);
   if (a.strided) {
     if constexpr (sizeof(R) == 8) {
       if (idx32) k_cumulant_fast<S, double, uint32_t, true><<<(unsigned)n_work * 4u, 128, 0, st>>>(a, work);
@@ -1837,8 +1878,9 @@ cudaError_t launch_fast(const StepArgs& a, const int32_t* work, int n_work, cuda
 template <class S, class R>
 cudaError_t launch_general(const StepArgs& a, const int32_t* work, int n_work, cudaStream_t st) {
   if (n_work <= 0) return cudaSuccess;
-  if (a.dense) k_cumulant_gen<S, R, true><<<(unsigned)n_work * 4u, 128, 0, st>>>(a, work);
-  else k_cumulant_gen<S, R, false><<<(unsigned)n_work * 4u, 128, 0, st>>>(a, work);
+  if (a.dense) k_cumulant_gen<S, R, true, false><<<(unsigned)n_work * 4u, 128, 0, st>>>(a, work);
+  else if (a.faces) k_cumulant_gen<S, R, false, true><<<(unsigned)n_work * 4u, 128, 0, st>>>(a, work);
+  else k_cumulant_gen<S, R, false, false><<<(unsigned)n_work * 4u, 128, 0, st>>>(a, work);
   return cudaGetLastError();
 }
 

@@ -91,3 +91,47 @@ def test_unpaired_arrays_keep_the_general_route(oal, kw):
     want, got = run(case, "f32", STEPS, post=True), run(case, "f32", STEPS, **kw)
     for a, b in zip(got, want):
         assert np.array_equal(a, b)
+
+
+def holed(case):
+    """The case's domain without some of its blocks: missing neighbours inside the domain."""
+    from openaerolab_alpha_01_b200.amr import neighbor_table
+    from openaerolab_alpha_01_b200.cases import Case
+    from openaerolab_alpha_01_b200.solver import BlockDomain
+    d = case.dom
+    keep = [i for i, c in enumerate(d.coords.tolist()) if c not in ([2, 2, 2], [4, 1, 3], [5, 5, 5])]
+    coords = np.ascontiguousarray(d.coords[keep])
+    dom = BlockDomain(d.bx_max, d.by_max, d.bz_max, coords, neighbor_table(coords, (d.bx_max, d.by_max, d.bz_max)),
+                      obstacle=None if d.obstacle is None else np.ascontiguousarray(d.obstacle[keep]))
+    return Case(case.name, dom, np.ascontiguousarray(case.rho[keep]), np.ascontiguousarray(case.vel[:, keep]), case.params)
+
+
+# the default face values come from the pull's address, every other option from the full face logic
+OPTIONS = [dict(), dict(inlet_turbulence=0.05, time_step_seed=3), dict(compressible_corr=1), dict(zwall_bc=1),
+           dict(zwall_bc=2), dict(ymin_wall_bc=1), dict(transverse_freestream=1, transverse_freestream_blend=0.4)]
+
+
+@pytest.mark.parametrize("storage", ["f32", "f64"])
+@pytest.mark.parametrize("options", OPTIONS, ids=lambda o: "-".join(o) or "default")
+@pytest.mark.parametrize("holes", [False, True])
+def test_face_values_match_the_ghost_filled_level(oal, storage, options, holes):
+    from openaerolab_alpha_01_b200.solver import Level
+    case = sphere_channel_case(40, 40, 40, diameter=8.0, centre_x=16.0, re=100.0, **options)
+    if holes:
+        case = holed(case)
+    r = np.random.default_rng(5)
+    case.vel = case.vel + 0.01 * r.standard_normal(case.vel.shape) * (case.dom.obstacle == 0)
+    case.params.compressible_corr = options.get("compressible_corr", 0)
+    got = run(case, storage, STEPS)
+    g = Geometry(case.dom)
+    L = Level(g, storage=storage)
+    L.init_equilibrium(case.rho, case.vel)
+    for _ in range(STEPS):
+        L.perform_timestep(case.params)
+    f, rho, vel = L.state()
+    force = L.forces()
+    for a, b in zip(got[:3], (f, rho.reshape(-1), vel.reshape(-1))):
+        assert np.max(np.abs(a - b)) < TOL[storage] * np.max(np.abs(b))
+    assert np.max(np.abs(got[3] - force)) <= 10 * TOL[storage] * max(np.max(np.abs(force)), 1e-2)
+    L.close()
+    g.close()
