@@ -2771,7 +2771,10 @@ struct BatchMember {
   BouzidiSet bz;  // linear Bouzidi boundary cells (oal_batch_set_bouzidi), pool block indices
 };
 
+constexpr size_t kStageKeep = size_t(64) << 20;
 struct oal_batch {
+  double* d_stage = nullptr;  // oal_batch_get_state
+  size_t stage_bytes = 0;
   int device = 0;
   int32_t storage = 0;
   int64_t R = 0, G = 0, M = 0;  // capacities: real blocks, ghost blocks, mask slots
@@ -3007,7 +3010,7 @@ void oal_batch_destroy(oal_batch* B) {
   for (int i = 0; i < 2; ++i) { cudaFree(B->f[i]); cudaFree(B->vel[i]); }
   cudaFree(B->rho); cudaFree(B->d_nbr); cudaFree(B->d_binfo); cudaFree(B->d_bflags); cudaFree(B->d_mslot);
   cudaFree(B->d_cmask); cudaFree(B->d_sponge); cudaFree(B->d_wdist); cudaFree(B->d_cases);
-  cudaFree(B->d_gentries); cudaFree(B->d_fast); cudaFree(B->d_general); cudaFree(B->d_seg);
+  cudaFree(B->d_stage); cudaFree(B->d_gentries); cudaFree(B->d_fast); cudaFree(B->d_general); cudaFree(B->d_seg);
   cudaFree(B->d_fast_rec); cudaFree(B->d_fcopy);
   cudaFree(B->d_part); cudaFree(B->d_forces); cudaFree(B->d_mm_part); cudaFree(B->d_mm);
   if (B->cap) cudaStreamDestroy(B->cap);
@@ -3331,12 +3334,28 @@ oal_status oal_batch_get_state(oal_batch* B, int32_t m, double* f, double* rho, 
   OAL_CUDA_TRY(cudaDeviceSynchronize());
   const BatchMember& M = B->mem[(size_t)m];
   const int64_t ncell = M.nb * 512;
-  double *df = nullptr, *dr = nullptr, *dv = nullptr;
+  // the doubles of one member on their way to the host: up to kStageKeep bytes in a buffer that the
+  // batch keeps (three allocations and three releases per member were a third of reading the fields of
+  // 16 members of 16^3 to 64^3 cells), more in one of its own
+  const size_t values = (size_t)ncell * ((f ? 27 : 0) + (rho ? 1 : 0) + (vel ? 3 : 0)), bytes = values * sizeof(double);
+  double* stage = nullptr;
   cudaError_t e = cudaSuccess;
-  if (f) e = cudaMalloc(&df, 27 * ncell * sizeof(double));
-  if (e == cudaSuccess && rho) e = cudaMalloc(&dr, ncell * sizeof(double));
-  if (e == cudaSuccess && vel) e = cudaMalloc(&dv, 3 * ncell * sizeof(double));
+  const bool keep = bytes <= kStageKeep;
+  if (keep && bytes > B->stage_bytes) {
+    cudaFree(B->d_stage);
+    B->d_stage = nullptr;
+    B->stage_bytes = 0;
+    e = cudaMalloc(&B->d_stage, bytes);
+    if (e == cudaSuccess) B->stage_bytes = bytes;
+  }
+  if (keep) stage = B->d_stage;
+  else e = cudaMalloc(&stage, bytes);
+  double *df = nullptr, *dr = nullptr, *dv = nullptr;
   if (e == cudaSuccess) {
+    double* p = stage;
+    if (f) { df = p; p += 27 * ncell; }
+    if (rho) { dr = p; p += ncell; }
+    if (vel) dv = p;
     switch (B->storage) {
       case OAL_STORE_F32: e = pool_export_t<float, float>(B, M, df, dr, dv); break;
       case OAL_STORE_F16_DEV: e = pool_export_t<__half, float>(B, M, df, dr, dv); break;
@@ -3347,11 +3366,10 @@ oal_status oal_batch_get_state(oal_batch* B, int32_t m, double* f, double* rho, 
   if (e == cudaSuccess && f) e = cudaMemcpy(f, df, 27 * ncell * sizeof(double), cudaMemcpyDeviceToHost);
   if (e == cudaSuccess && rho) e = cudaMemcpy(rho, dr, ncell * sizeof(double), cudaMemcpyDeviceToHost);
   if (e == cudaSuccess && vel) e = cudaMemcpy(vel, dv, 3 * ncell * sizeof(double), cudaMemcpyDeviceToHost);
-  cudaFree(df); cudaFree(dr); cudaFree(dv);
+  if (!keep) cudaFree(stage);
   if (e != cudaSuccess) return set_error(OAL_E_CUDA, "batch_get_state: %s", cudaGetErrorString(e));
   return OAL_OK;
 }
-
 oal_status oal_batch_get_forces(oal_batch* B, int32_t m, double out[3]) {
   if (!B || !out || m < 0 || m >= B->max_members || !B->mem[(size_t)m].active) return set_error(OAL_E_INVALID_ARG, "no such member");
   OAL_CUDA_TRY(cudaSetDevice(B->device));
