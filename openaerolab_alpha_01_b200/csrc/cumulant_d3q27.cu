@@ -422,14 +422,20 @@ __global__ void __launch_bounds__(128, sizeof(R) == 8 ? 2 : 4) k_parent_fill(con
   const int32_t id0 = nodes[lane], id1 = nodes[lane + 32];
   const uint2 mem = lane < 8 ? P.grp_mem[(int64_t)g * 8 + lane] : make_uint2(0u, 0u);
   R v[4][4][4];
+  if (cubic && all) {
 #pragma unroll
-  for (int i = 0; i < 64; ++i) {
-    const int a = i >> 4, b = (i >> 2) & 3, c = i & 3;
-    const int32_t id = __shfl_sync(0xffffffffu, i < 32 ? id0 : id1, i & 31);
-    // outside the cubic range only the bracket's corners count
-    const bool outer = a == 0 || a == 3 || b == 0 || b == 3 || c == 0 || c == 3;
-    if (outer && !cubic) v[a][b][c] = R(0);
-    else v[a][b][c] = (all || id >= 0) ? vals[(int64_t)id * 32] : anchor;
+    for (int i = 0; i < 64; ++i)
+      v[i >> 4][(i >> 2) & 3][i & 3] = vals[(int64_t)__shfl_sync(0xffffffffu, i < 32 ? id0 : id1, i & 31) * 32];
+  } else {
+#pragma unroll
+    for (int i = 0; i < 64; ++i) {
+      const int a = i >> 4, b = (i >> 2) & 3, c = i & 3;
+      const int32_t id = __shfl_sync(0xffffffffu, i < 32 ? id0 : id1, i & 31);
+      // outside the cubic range only the bracket's corners count
+      const bool outer = a == 0 || a == 3 || b == 0 || b == 3 || c == 0 || c == 3;
+      if (outer && !cubic) v[a][b][c] = R(0);
+      else v[a][b][c] = (all || id >= 0) ? vals[(int64_t)id * 32] : anchor;
+    }
   }
   R acc[2][2][2] = {};
 #pragma unroll
@@ -1692,16 +1698,19 @@ __global__ void __launch_bounds__(128) k_restrict(const RestrictArgs r) {
   R avg[kQ27];
 #pragma unroll
   for (int k = 0; k < kQ27; ++k) avg[k] = R(0);
+  // the solid children, before the first population is read: bits 2 i and 2 i + 1 of the pairs
+  uint32_t solid = 0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    if (r.cbflags[cblk[i]] & BF_NEAR_SOLID) {
+      const uint32_t* m = r.ccmask + (int64_t)r.cmslot[cblk[i]] * kCells + ccell[i];
+      solid |= ((m[0] >> 13) & 1u) << (2 * i) | ((m[1] >> 13) & 1u) << (2 * i + 1);
+    }
   int fluid = 0;
 #pragma unroll 1
   for (int i = 0; i < 4; ++i) {
     const int cb = cblk[i];
-    bool f0 = true, f1 = true;
-    if (r.cbflags[cb] & BF_NEAR_SOLID) {
-      const uint32_t* m = r.ccmask + (int64_t)r.cmslot[cb] * kCells + ccell[i];
-      f0 = !((m[0] >> 13) & 1u);
-      f1 = !((m[1] >> 13) & 1u);
-    }
+    const bool f0 = !((solid >> (2 * i)) & 1u), f1 = !((solid >> (2 * i + 1)) & 1u);
     fluid += (int)f0 + (int)f1;
     const Pair* c = reinterpret_cast<const Pair*>(cf + (int64_t)cb * (27 * kCells) + ccell[i]);
 #pragma unroll

@@ -438,7 +438,7 @@ struct Overlap {
 
 // The captured steps that start from one parity of the ping-pong buffers. A level keeps one per
 // parity: an odd number of steps ends on the other one, and with a single graph every second call
-// re-captured (a channel of 200 x 88 x 104 in FP32, 5 steps a call: 684 us against 560 us).
+// re-captured (a channel of 200 x 88 x 104 in FP32, 5 steps a call: 673 us against 525 us).
 struct GraphCache {
   cudaGraphExec_t exec = nullptr;
   cudaGraph_t graph = nullptr;
