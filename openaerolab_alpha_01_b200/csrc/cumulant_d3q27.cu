@@ -212,9 +212,10 @@ __global__ void __launch_bounds__(kNodeThreads) k_parent_nodes(const ParentView 
 template <class S, class R>
 cudaError_t launch_parent_nodes(const StepArgs& a, cudaStream_t st) {
   const ParentView& P = a.par;
-  if (P.n_nodes <= 0) return cudaSuccess;
-  k_parent_nodes<S, R><<<(unsigned)((P.n_nodes + kNodeThreads - 1) / kNodeThreads), kNodeThreads, 0, st>>>(
-      P, P.nodes, P.n_nodes, static_cast<R*>(const_cast<void*>(P.node_vals)), (a.p0.flags & CF_COMPRESSIBLE) != 0);
+  const ParentFill& F = *P.fill;
+  if (F.n_nodes <= 0) return cudaSuccess;
+  k_parent_nodes<S, R><<<(unsigned)((F.n_nodes + kNodeThreads - 1) / kNodeThreads), kNodeThreads, 0, st>>>(
+      P, F.nodes, F.n_nodes, static_cast<R*>(const_cast<void*>(P.node_vals)), (a.p0.flags & CF_COMPRESSIBLE) != 0);
   return cudaGetLastError();
 }
 
@@ -384,11 +385,11 @@ __device__ __noinline__ void node_macros(const R* vals, int pnx, int pny, int pn
 // for the macros: 290 + 124 us per substep of the two-level sphere channel (256 x 128 x 128, refined
 // box 96 x 64 x 64, FP16; 131,000 ghost cells).
 template <class S, class R>
-__global__ void __launch_bounds__(128, sizeof(R) == 8 ? 2 : 4) k_parent_fill(const ParentView P, S* __restrict__ f, int32_t n_real, bool comp) {
+__global__ void __launch_bounds__(128, sizeof(R) == 8 ? 2 : 4) k_parent_fill(const ParentView P, const ParentFill F, S* __restrict__ f, int32_t n_real, bool comp) {
   const int32_t g = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (g >= P.n_groups) return;
-  const int4 gx = P.grp_xyz[g];
-  const int32_t* nodes = P.grp_nodes + (int64_t)g * 64;
+  if (g >= F.n_groups) return;
+  const int4 gx = F.grp_xyz[g];
+  const int32_t* nodes = F.grp_nodes + (int64_t)g * 64;
   const R* __restrict__ vals = static_cast<const R*>(P.node_vals) + lane;
   const bool cubic = (gx.w & GF_CUBIC) != 0, all = (gx.w & GF_ALL_NODES) != 0;
   // per axis and parity of the fine coordinate the weights of the four nodes, one per lane (24), then
@@ -420,7 +421,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 8 ? 2 : 4) k_parent_fill(con
   // the 64 ids in two loads a lane, then every record read of the group in flight at once: a warp
   // waits for two trips to memory (per-quad index loads and 16 records at a time: eight, 112 us)
   const int32_t id0 = nodes[lane], id1 = nodes[lane + 32];
-  const uint2 mem = lane < 8 ? P.grp_mem[(int64_t)g * 8 + lane] : make_uint2(0u, 0u);
+  const uint2 mem = lane < 8 ? F.grp_mem[(int64_t)g * 8 + lane] : make_uint2(0u, 0u);
   R v[4][4][4];
   // a full stencil (all groups away from domain faces and holes) without the test and select per record;
   // with k_restrict's masks ahead of its reads 1545 -> 1466 us for two coarse steps of the same channel
@@ -487,9 +488,10 @@ __global__ void __launch_bounds__(128, sizeof(R) == 8 ? 2 : 4) k_parent_fill(con
 
 template <class S, class R>
 cudaError_t launch_parent_fill(const StepArgs& a, cudaStream_t st) {
-  if (a.par.n_groups <= 0) return cudaSuccess;
-  k_parent_fill<S, R><<<(unsigned)((a.par.n_groups + 3) / 4), 128, 0, st>>>(
-      a.par, const_cast<S*>(static_cast<const S*>(a.f_in)), a.n_blocks, (a.p0.flags & CF_COMPRESSIBLE) != 0);
+  const ParentFill& F = *a.par.fill;
+  if (F.n_groups <= 0) return cudaSuccess;
+  k_parent_fill<S, R><<<(unsigned)((F.n_groups + 3) / 4), 128, 0, st>>>(
+      a.par, F, const_cast<S*>(static_cast<const S*>(a.f_in)), a.n_blocks, (a.p0.flags & CF_COMPRESSIBLE) != 0);
   return cudaGetLastError();
 }
 

@@ -723,7 +723,7 @@ static cudaError_t launch_step_t(const oal_geometry* g, const StepArgs& a0, Step
       // (domain faces and slip images, which read the records too)
       if ((r = launch_parent_nodes<S, R>(a, s)) != cudaSuccess) return r;
       if ((r = launch_parent_fill<S, R>(a, s)) != cudaSuccess) return r;
-      return launch_fill_ghosts<S, R>(a, a.par.rest, a.par.n_rest, s);
+      return launch_fill_ghosts<S, R>(a, a.par.fill->rest, a.par.fill->n_rest, s);
     }
     if (!fl) return launch_fill_ghosts<S, R>(a, g->d_gentries, g->n_gentries, s);
     if ((r = launch_fill_copy<S, R>(a, fl->copy, fl->n_copy, s)) != cudaSuccess) return r;
@@ -2216,6 +2216,7 @@ struct AmrLevel {
   uint2* d_grp_mem = nullptr;
   uint2* d_rest = nullptr;
   int64_t n_rest = 0;
+  ParentFill fill{};              // the same for the launchers (set by amr_step)
   // populations and velocity before the level's step: the step's input buffers, which no launch of
   // the coarse step rewrites (set by amr_step)
   const void* f_old = nullptr;
@@ -2306,14 +2307,15 @@ static oal_status amr_step(oal_amr* A, int l, const std::vector<CaseParams>& cps
     v.use_temporal = 1;  // TEMPORAL_INTERPOLATION (config_loader.jl:90)
     v.node_map = me.d_node_map;
     v.node_vals = me.d_node_vals;
-    v.nodes = me.d_nodes;
-    v.n_nodes = me.n_nodes;
-    v.grp_xyz = me.d_grp_xyz;
-    v.grp_nodes = me.d_grp_nodes;
-    v.grp_mem = me.d_grp_mem;
-    v.n_groups = me.n_groups;
-    v.rest = me.d_rest;
-    v.n_rest = me.n_rest;
+    me.fill.nodes = me.d_nodes;
+    me.fill.n_nodes = me.n_nodes;
+    me.fill.grp_xyz = me.d_grp_xyz;
+    me.fill.grp_nodes = me.d_grp_nodes;
+    me.fill.grp_mem = me.d_grp_mem;
+    me.fill.n_groups = me.n_groups;
+    me.fill.rest = me.d_rest;
+    me.fill.n_rest = me.n_rest;
+    v.fill = &me.fill;
     L->par = v;
   }
   CaseParams cp = cps[(size_t)l];
