@@ -485,7 +485,8 @@ struct oal_level {
   float* s_out = nullptr;
   double* s_part = nullptr;
   double* s_sum = nullptr;
-  uint32_t bz_gen = 0;      // bumped by every oal_level_set_bouzidi (hierarchy graphs compare it)
+  uint32_t settings_gen = 0;  // bumped by settings_changed: what a hierarchy's captured steps hold of the
+                              // level besides its parameters (Bouzidi cells, outlet, launch tuning)
   // variable nu_sgs from Pi_neq: the post-collision non-equilibrium stress of the previous step,
   // 6 components x n_blocks x 512 in the compute type, refreshed in place by the general kernel
   void* pi_neq = nullptr;
@@ -1566,6 +1567,13 @@ static void release_graph(oal_level* L) {
   L->gc[1].release();
 }
 
+// A setting that captured launches hold by value or by pointer is about to change: the level's own
+// graphs go, a hierarchy's are found stale by the generation.
+static void settings_changed(oal_level* L) {
+  release_graph(L);
+  ++L->settings_gen;
+}
+
 void oal_level_destroy(oal_level* L) {
   if (!L) return;
   if (L->kbc) {
@@ -1844,8 +1852,7 @@ oal_status oal_level_set_bouzidi(oal_level* L, int32_t n_cells, const int32_t* c
   if (L->kbc) return set_error(OAL_E_UNSUPPORTED, "linear Bouzidi walls are a D3Q27 level path");
   OAL_CUDA_TRY(cudaSetDevice(L->g->device));
   OAL_CUDA_TRY(cudaDeviceSynchronize());  // a step in flight may still read the old set
-  release_graph(L);
-  ++L->bz_gen;
+  settings_changed(L);
   return bouzidi_upload(&L->bz, L->storage, L->g->nb, 0, n_cells, cell_block, cell_x, cell_y, cell_z, q_half,
                         q_min_threshold, ff_fallback, limiter_rel_cap, limiter_abs_cap);
 }
@@ -2074,6 +2081,9 @@ oal_status oal_level_set_nscbc(oal_level* L, const oal_nscbc_params* np) {
     for (int32_t b = 0; b < g->nb; ++b)
       if (np->all_blocks || g->h_binfo[(size_t)b].x == bxmax) list.push_back(b);
   }
+  OAL_CUDA_TRY(cudaDeviceSynchronize());  // a step in flight may still read the old list
+  settings_changed(L);
+  L->nscbc = oal_nscbc_params{};
   cudaFree(L->d_nscbc_blocks);
   L->d_nscbc_blocks = nullptr;
   L->n_nscbc = 0;
@@ -2083,7 +2093,6 @@ oal_status oal_level_set_nscbc(oal_level* L, const oal_nscbc_params* np) {
     L->n_nscbc = (int32_t)list.size();
   }
   L->nscbc = *np;
-  release_graph(L);  // the captured steps hold the old setting
   return OAL_OK;
 }
 
@@ -2095,7 +2104,7 @@ oal_status oal_level_set_tuning(oal_level* L, int32_t key, int64_t value) {
     return set_error(OAL_E_INVALID_ARG, "tuning key %d: value %lld", key, (long long)value);
   if (*slot != (int32_t)value) {
     *slot = (int32_t)value;
-    release_graph(L);  // the captured launches hold the old value
+    settings_changed(L);
   }
   return OAL_OK;
 }
@@ -2228,13 +2237,17 @@ struct oal_amr {
   int32_t storage = 0;
   std::vector<AmrLevel> lv;
   cudaStream_t cap = nullptr;
-  // the captured coarse steps, by the coarsest level's starting parity (as GraphCache)
+  // the captured coarse steps, by the coarsest level's starting parity (as GraphCache); what they hold
+  // of each level
+  struct Held {
+    oal_step_params p;
+    uint32_t settings;  // oal_level::settings_gen
+  };
   struct Graph {
     cudaGraphExec_t exec = nullptr;
     cudaGraph_t graph = nullptr;
     int32_t n = 0;
-    std::vector<oal_step_params> p;
-    std::vector<uint32_t> bz;  // the levels' Bouzidi generations the graph was captured with
+    std::vector<Held> held;
   } gr[2];
 };
 
@@ -2632,12 +2645,14 @@ oal_status oal_amr_advance(oal_amr* A, const oal_step_params* params, int32_t n,
   }
   const int start = A->lv[0].L->parity;
   oal_amr::Graph& G = A->gr[start];
-  bool hit = G.exec && G.n == n && (int)G.p.size() == nl;
+  bool hit = G.exec && G.n == n && (int)G.held.size() == nl;
   for (int l = 0; hit && l < nl; ++l) {
-    oal_step_params a = params[l], b = G.p[(size_t)l];
+    const oal_amr::Held& h = G.held[(size_t)l];
+    const oal_level* L = A->lv[(size_t)l].L;
+    oal_step_params a = params[l], b = h.p;
     a.time_step_seed = b.time_step_seed = 0;
     hit = std::memcmp(&a, &b, sizeof a) == 0 && !(cps[(size_t)l].flags & CF_INLET_NOISE) &&
-          G.bz.size() == (size_t)nl && G.bz[(size_t)l] == A->lv[(size_t)l].L->bz_gen;
+          h.settings == L->settings_gen;
   }
   std::vector<int> parities((size_t)nl);
   for (int l = 0; l < nl; ++l) parities[(size_t)l] = A->lv[(size_t)l].L->parity;
@@ -2655,9 +2670,10 @@ oal_status oal_amr_advance(oal_amr* A, const oal_step_params* params, int32_t n,
     e = cudaGraphInstantiate(&exec, graph, 0);
     if (e != cudaSuccess) { cudaGraphDestroy(graph); cudaGetLastError(); return set_error(OAL_E_CUDA, "graph instantiate: %s", cudaGetErrorString(e)); }
     G.exec = exec; G.graph = graph; G.n = n;
-    G.p.assign(params, params + nl);
-    G.bz.resize((size_t)nl);
-    for (int l = 0; l < nl; ++l) G.bz[(size_t)l] = A->lv[(size_t)l].L->bz_gen;
+    for (int l = 0; l < nl; ++l) {
+      const oal_level* L = A->lv[(size_t)l].L;
+      G.held.push_back({params[l], L->settings_gen});
+    }
   }
   OAL_CUDA_TRY(cudaGraphLaunch(G.exec, static_cast<cudaStream_t>(stream)));
   // level l takes n * 2^l steps: only the coarsest level can end on the other buffer

@@ -66,3 +66,48 @@ def test_odd_hierarchy_calls_equal_single_steps(oal, calls):
             assert np.array_equal(x, y)
     for t in trees:
         t.close()
+
+
+def two_levels(n_trees=1):
+    from openaerolab_alpha_01_b200.amr import Hierarchy, blocks_in_box, level_taus, refine
+    from openaerolab_alpha_01_b200.solver import build_box, default_step_params
+    coarse = build_box(5, 4, 4)
+    doms = [coarse, refine(coarse, blocks_in_box(coarse, (16, 8, 8), (24, 24, 24)))]
+    P = [default_step_params(tau=t, c_wale=0.2, u_inlet=0.05) for t in level_taus(0.53, 2)]
+    trees = [Hierarchy(doms, storage="f32") for _ in range(n_trees)]
+    r = np.random.default_rng(3)
+    for l, d in enumerate(doms):
+        vel = 0.05 + 0.005 * r.standard_normal((3, d.n_blocks, 512))
+        for t in trees:
+            t.level(l).init_equilibrium(np.ones((d.n_blocks, 512)), vel)
+    return doms, P, trees
+
+
+# (coarse steps, outlet setting before them): on, changed and off between calls of counts that have a
+# captured graph from either buffer
+ON, CHANGED, OFF = dict(p_target=1.0 / 3.0), dict(p_target=0.34, sigma_relax=0.5, all_blocks=True), dict(enabled=False)
+OUTLET = [[(1, None), (1, None), (1, ON), (1, None), (1, CHANGED), (1, None), (1, OFF), (1, None)],
+          [(2, ON), (2, None), (2, CHANGED), (2, OFF), (2, None), (2, ON)],
+          [(3, ON), (1, None), (3, CHANGED), (3, None), (1, OFF), (3, None), (3, None)]]
+
+
+@pytest.mark.parametrize("calls", OUTLET)
+def test_hierarchy_calls_see_the_outlet_as_it_is_set(oal, calls):
+    from openaerolab_alpha_01_b200.amr import Hierarchy
+    doms, P, (tree,) = two_levels()
+    outlet = OFF
+    for n, change in calls:
+        if change is not None:
+            outlet = change
+            tree.level(0).set_nscbc(**change)
+        fresh = Hierarchy(doms, storage="f32")  # the same state and outlet, no captured steps
+        for l in range(2):
+            fresh.level(l).set_state(*tree.level(l).state())
+        fresh.level(0).set_nscbc(**outlet)
+        tree.advance(P, n)
+        fresh.advance(P, n)
+        for l in range(2):
+            for x, y in zip(tree.level(l).state(), fresh.level(l).state()):
+                assert np.array_equal(x, y), (n, change, l)
+        fresh.close()
+    tree.close()
