@@ -2238,10 +2238,12 @@ struct oal_amr {
   std::vector<AmrLevel> lv;
   cudaStream_t cap = nullptr;
   // the captured coarse steps, by the coarsest level's starting parity (as GraphCache); what they hold
-  // of each level
+  // of each level, and the level's view of its parent after the last captured step
   struct Held {
     oal_step_params p;
     uint32_t settings;  // oal_level::settings_gen
+    int parity;
+    ParentView par;
   };
   struct Graph {
     cudaGraphExec_t exec = nullptr;
@@ -2651,8 +2653,9 @@ oal_status oal_amr_advance(oal_amr* A, const oal_step_params* params, int32_t n,
     const oal_level* L = A->lv[(size_t)l].L;
     oal_step_params a = params[l], b = h.p;
     a.time_step_seed = b.time_step_seed = 0;
+    // the finer levels' parities too: a call on a level of its own may have turned one
     hit = std::memcmp(&a, &b, sizeof a) == 0 && !(cps[(size_t)l].flags & CF_INLET_NOISE) &&
-          h.settings == L->settings_gen;
+          h.settings == L->settings_gen && h.parity == L->parity;
   }
   std::vector<int> parities((size_t)nl);
   for (int l = 0; l < nl; ++l) parities[(size_t)l] = A->lv[(size_t)l].L->parity;
@@ -2672,8 +2675,15 @@ oal_status oal_amr_advance(oal_amr* A, const oal_step_params* params, int32_t n,
     G.exec = exec; G.graph = graph; G.n = n;
     for (int l = 0; l < nl; ++l) {
       const oal_level* L = A->lv[(size_t)l].L;
-      G.held.push_back({params[l], L->settings_gen});
+      G.held.push_back({params[l], L->settings_gen, L->parity, L->par});
     }
+  }
+  // the levels' views of their parents, which a step of a level on its own interpolates from, as these
+  // steps leave them; graphs such a step captured hold an older view
+  for (int l = 1; l < nl; ++l) {
+    oal_level* L = A->lv[(size_t)l].L;
+    L->par = G.held[(size_t)l].par;
+    release_graph(L);
   }
   OAL_CUDA_TRY(cudaGraphLaunch(G.exec, static_cast<cudaStream_t>(stream)));
   // level l takes n * 2^l steps: only the coarsest level can end on the other buffer

@@ -111,3 +111,26 @@ def test_hierarchy_calls_see_the_outlet_as_it_is_set(oal, calls):
                 assert np.array_equal(x, y), (n, change, l)
         fresh.close()
     tree.close()
+
+
+@pytest.mark.parametrize("calls", [[1, 1, 1], [1, 1, 1, 1, 1], [3, 3, 3]])
+def test_hierarchy_with_steps_of_a_refined_level_between(oal, calls):
+    """A refined level stepped on its own interpolates from the parent as the last coarse step left it, whether
+    that step was captured or replayed; the coarse steps after it start from the buffer it ended on."""
+    _, P, (a, b) = two_levels(2)
+    for n in calls:
+        a.advance(P, n)
+    b.advance(P, sum(calls))
+    for _ in range(2):
+        for t in (a, b):
+            t.level(1).perform_timestep(P[1])
+        a.level(1).execute_timestep_batch(P[1], 2)
+        for _ in range(2):
+            b.level(1).perform_timestep(P[1])
+        a.advance(P, 1)
+        b.advance(P, 1)
+        for l in range(2):
+            for x, y in zip(a.level(l).state(), b.level(l).state()):
+                assert np.array_equal(x, y)
+    a.close()
+    b.close()
