@@ -567,16 +567,22 @@ __device__ __forceinline__ void solve_lambdas(const Tables& T, float rho, float 
     bool cold = la[0] != la[0];
     if (cold) poly_start();
     for (int it = 0; it < KBC_NEWTON_MAX; ++it) {
-      if (!eq_pops(rho, la, fe)) break;
+      const bool held = eq_pops(rho, la, fe);
       NewtonPass np;
-      float r[13];
-      const float res = np.residual(fe, rho, ux, uy, uz, r);
-      if (res < TOL_SQ) return;
-      if (!cold && it == 0 && res > warm_gate * TOL_SQ) {
-        // staleness gate on the warm start (physics_utils.jl:603-634)
+      float r[13], res = 0.0f;
+      if (held) {
+        res = np.residual(fe, rho, ux, uy, uz, r);
+        if (res < TOL_SQ) return;
+      }
+      if (!held || (!cold && it == 0 && res > warm_gate * TOL_SQ)) {
+        // staleness gate on the warm start (physics_utils.jl:603-634): a stale one, and one with some
+        // |lda| that may exceed 20, gives way to the polynomial start; the sweeps, which clamp, take over
+        // where that one leaves the range too
+        const bool warm = !cold;
         poly_start();
         cold = true;
-        continue;
+        if (warm) continue;
+        break;
       }
       float H[91];
       np.hess(H);

@@ -358,3 +358,36 @@ def test_fast_math_within_tolerance(env, name):
     assert np.array_equal(np.isnan(lam), np.isnan(ora.lam))
     fin = np.isfinite(lam)
     assert float(np.max(np.abs(lam[fin] - ora.lam[fin])) / np.max(np.abs(ora.lam[fin]))) < 2e-3
+
+
+# cached multipliers whose |lda| bound exceeds 20: one component, all of them, of either sign, and beyond it by far
+STRAY = {"constant": {0: 25.0}, "linear": {1: 8.0}, "stress": {4: 3.0, 7: -6.0}, "flux": {10: 1.2, 12: -1.2},
+         "all": {m: 4.0 * (-1) ** m for m in range(13)}, "far": {5: 1e6}}
+
+
+@pytest.mark.parametrize("name", sorted(STRAY))
+def test_stray_cached_multipliers_start_over(env, name):
+    """The fast step gives a warm start whose exponentials may leave the clamp's range up for the polynomial
+    start, so cells with such multipliers step to the same bits as cells without any."""
+    _, solver = env
+    dom = solver.build_box(2, 1, 1, periodic=(True, True, True))
+    rho, vel = smooth_fields(dom, u0=0.1, seed=6)
+    p = solver.default_entropic_params(tau=0.53, c_wale=0.2)
+    got = []
+    for stray in (True, False):
+        geom = solver.Geometry(dom)
+        lvl = solver.Level(geom, "entropic")
+        lvl.init_equilibrium(rho, vel)
+        lam = np.full((13, dom.n_blocks, 512), np.nan, np.float32)
+        if stray:
+            lam[:, :, ::3] = 0.0
+            for m, v in STRAY[name].items():
+                lam[m, :, ::3] = v
+        lvl.lambda_cache(lam)
+        lvl.step(p)
+        got.append((*lvl.state(), lvl.lambda_cache()))
+        lvl.close()
+        geom.close()
+    assert np.all(np.isfinite(got[1][3]))
+    for a, b in zip(*got):
+        assert same_bits(a, b)
