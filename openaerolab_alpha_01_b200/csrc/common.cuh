@@ -76,7 +76,8 @@ enum CaseFlags : uint32_t {
   CF_BOUZIDI = 1u << 19,     // linear Bouzidi correction after the step (the step itself is full-way)
   CF_GENERAL_RATES = 1u << 20, // omega_bulk, omega3 or omega4 differs from 1 (the configuration default)
   CF_SGS_PI = 1u << 21,        // variable nu_sgs from the stored post-collision Pi_neq
-  CF_SGS_DYNAMIC = 1u << 22    // variable nu_sgs from the Germano-Lilly dynamic coefficient
+  CF_SGS_DYNAMIC = 1u << 22,   // variable nu_sgs from the Germano-Lilly dynamic coefficient
+  CF_BEYOND = 1u << 23         // caller-owned arrays: some block reaches beyond the domain's cell extent
 };
 
 struct CaseParams {

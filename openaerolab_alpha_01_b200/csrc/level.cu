@@ -382,6 +382,7 @@ struct oal_geometry {
   int32_t n_fast_in = 0;           // the first n_fast_in fast blocks read no ghost slot
   int32_t* d_plain = nullptr;      // every other block: fast blocks at domain faces, general blocks
   int32_t n_plain = 0;
+  bool beyond = false;             // some block reaches beyond the cell extent (no multiple of 8)
   int32_t* d_general = nullptr;    // blocks for the general kernel
   int32_t n_fast = 0, n_general = 0;
   // ghost fill split by face conditions (one entry per key of fill_key_of, kept until the
@@ -1118,6 +1119,9 @@ oal_status oal_geometry_create(const oal_geometry_desc* d, int32_t device, oal_g
     if (interior) bflags[(size_t)b] |= BF_INTERIOR;
   }
   auto* g = new oal_geometry();
+  for (const int4& c : binfo)
+    g->beyond = g->beyond || c.x < 1 || c.y < 1 || c.z < 1 || (int64_t)c.x * kBS > d->nx_global ||
+                (int64_t)c.y * kBS > d->ny_global || (int64_t)c.z * kBS > d->nz_global;
   g->device = device;
   g->nb = d->n_blocks; g->nx = d->nx_global; g->ny = d->ny_global; g->nz = d->nz_global;
 
@@ -1381,6 +1385,7 @@ oal_status oal_stream_collide(const oal_geometry* g, const oal_level_fields* fl,
   a.v_bstride = 512; a.v_cstride = fl->vel_comp_stride > 0 ? fl->vel_comp_stride : 512 * (int64_t)g->nb;
   a.force_part = g->d_force_part;
   a.faces = 1;
+  if (g->beyond) cp.flags |= CF_BEYOND;
   a.p0 = cp;
   a.flags_any = cp.flags;
   cudaStream_t st = static_cast<cudaStream_t>(stream);

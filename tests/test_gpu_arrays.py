@@ -135,3 +135,35 @@ def test_face_values_match_the_ghost_filled_level(oal, storage, options, holes):
     assert np.max(np.abs(got[3] - force)) <= 10 * TOL[storage] * max(np.max(np.abs(force)), 1e-2)
     L.close()
     g.close()
+
+
+class ShortDomain:
+    """A block domain whose cell extent ends inside its last blocks."""
+
+    def __init__(self, dom, shape):
+        self.dom, self.shape = dom, shape
+
+    def __getattr__(self, name):
+        return getattr(self.dom, name)
+
+
+@pytest.mark.parametrize("storage", ["f32", "f64"])
+@pytest.mark.parametrize("shape", [(37, 40, 40), (40, 33, 40), (40, 40, 38), (36, 35, 39)])
+def test_face_values_of_extents_inside_a_block(oal, storage, shape):
+    from openaerolab_alpha_01_b200.solver import Level
+    case = sphere_channel_case(40, 40, 40, diameter=8.0, centre_x=16.0, re=100.0)
+    case.dom = ShortDomain(case.dom, shape)
+    r = np.random.default_rng(5)
+    case.vel = case.vel + 0.01 * r.standard_normal(case.vel.shape) * (case.dom.obstacle == 0)
+    case.params.compressible_corr = 0
+    got = run(case, storage, STEPS)
+    g = Geometry(case.dom)
+    L = Level(g, storage=storage)
+    L.init_equilibrium(case.rho, case.vel)
+    for _ in range(STEPS):
+        L.perform_timestep(case.params)
+    f, rho, vel = L.state()
+    for a, b in zip(got[:3], (f, rho.reshape(-1), vel.reshape(-1))):
+        assert np.max(np.abs(a - b)) < TOL[storage] * np.max(np.abs(b))
+    L.close()
+    g.close()
