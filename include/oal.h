@@ -487,7 +487,8 @@ oal_status oal_batch_get_state(oal_batch* B, int32_t member, double* f, double* 
 oal_status oal_batch_get_forces(oal_batch* B, int32_t member, double out[3]);
 oal_status oal_batch_mass_momentum(oal_batch* B, int32_t member, double out[4]);
 /* Pool usage: out = {members, real blocks used, ghost blocks used, mask blocks used,
- * real capacity, ghost capacity, mask capacity, device bytes}. */
+ * real capacity, ghost capacity, mask capacity, device bytes}. The device bytes include the buffer
+ * that oal_batch_get_state keeps for the batch's lifetime (at most 64 MB, the largest state read). */
 oal_status oal_batch_info(const oal_batch* B, int64_t out[8]);
 /* Blocks one member of this geometry occupies: out = {real, ghost, mask}. */
 oal_status oal_geometry_blocks(const oal_geometry* g, int64_t out[3]);

@@ -3377,9 +3377,11 @@ oal_status oal_batch_get_state(oal_batch* B, int32_t m, double* f, double* rho, 
   if (keep && bytes > B->stage_bytes) {
     cudaFree(B->d_stage);
     B->d_stage = nullptr;
+    B->bytes -= (int64_t)B->stage_bytes;
     B->stage_bytes = 0;
     e = cudaMalloc(&B->d_stage, bytes);
     if (e == cudaSuccess) B->stage_bytes = bytes;
+    B->bytes += (int64_t)B->stage_bytes;
   }
   if (keep) stage = B->d_stage;
   else e = cudaMalloc(&stage, bytes);
@@ -3403,6 +3405,7 @@ oal_status oal_batch_get_state(oal_batch* B, int32_t m, double* f, double* rho, 
   if (e != cudaSuccess) return set_error(OAL_E_CUDA, "batch_get_state: %s", cudaGetErrorString(e));
   return OAL_OK;
 }
+
 oal_status oal_batch_get_forces(oal_batch* B, int32_t m, double out[3]) {
   if (!B || !out || m < 0 || m >= B->max_members || !B->mem[(size_t)m].active) return set_error(OAL_E_INVALID_ARG, "no such member");
   OAL_CUDA_TRY(cudaSetDevice(B->device));

@@ -148,3 +148,20 @@ def test_member_of_a_pool_past_2_31_elements_matches_alone(oal):
     assert np.array_equal(B.state(m)[0], f)
     assert np.array_equal(B.forces(m), force) and np.array_equal(B.mass_momentum(m), mm)
     B.close(); g.close()
+
+
+def test_device_bytes_include_the_kept_read_back_buffer(oal):
+    cases = [taylor_green_case(16, u0=0.05, re=100.0, c_wale=0.0), taylor_green_case(24, u0=0.05, re=100.0, c_wale=0.0),
+             taylor_green_case(80, u0=0.05, re=100.0, c_wale=0.0)]
+    geoms = [Geometry(c.dom) for c in cases]
+    B = Batch(storage="f16", max_real_blocks=1100, max_ghost_blocks=8, max_mask_blocks=8, max_members=4)
+    ids = [B.add(g, c.params, c.rho, c.vel) for g, c in zip(geoms, cases)]
+    pool = B.info()["bytes"]
+    doubles = lambda edge: 31 * 8 * edge ** 3  # noqa: E731
+    # the first reads, a larger one, a smaller one again, and one beyond 64 MB, which keeps nothing
+    for m, kept in ((0, doubles(16)), (1, doubles(24)), (0, doubles(24)), (2, doubles(24))):
+        B.state(ids[m])
+        assert B.info()["bytes"] == pool + kept
+    B.close()
+    for g in geoms:
+        g.close()
