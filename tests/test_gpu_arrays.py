@@ -24,22 +24,23 @@ def weights():
     return np.array([(8 / 27, 2 / 27, 1 / 54, 1 / 216)[int(np.abs(k).sum())] for k in c])
 
 
-def run(case, storage, steps, off=0, block_stride=512, pad=0, post=False):
+def run(case, storage, steps, off=0, block_stride=512, pad=0, post=False, dir_stride=None, svv=(0.0, 0.0)):
     """The case's populations, density, velocity and force after `steps`, in caller-owned arrays that
-    start `off` elements into their buffers, with `pad` extra elements between directions."""
+    start `off` elements into their buffers, with `pad` extra elements between directions (or directions
+    `dir_stride` apart), the spectral-viscosity filter of strengths `svv` after each."""
     import torch
     dt = {"f32": torch.float32, "f64": torch.float64, "f16": torch.float16, "bf16": torch.bfloat16}[storage]
     mt = torch.float64 if storage == "f64" else torch.float32
     g, nb = Geometry(case.dom), case.dom.n_blocks
-    kst = block_stride * nb + pad
+    kst = dir_stride or block_stride * nb + pad
     w = weights()
     c = np.stack(np.meshgrid(*(np.arange(3) - 1,) * 3, indexing="ij"), -1).reshape(27, 3)[:, ::-1]  # x fastest
     cu = np.tensordot(c.astype(float), case.vel, 1)
     f0 = w[:, None, None] * case.rho * (1 + 3 * cu + 4.5 * cu ** 2 - 1.5 * (case.vel ** 2).sum(0))
     if storage in ("f16", "bf16"):
         f0 = f0 / w[:, None, None] - 1.0
-    size = 27 * kst + off
-    buf = [torch.zeros(size, dtype=dt, device="cuda") for _ in range(3)]
+    size = max(27 * kst, (nb - 1) * block_stride + 26 * kst + 512) + off
+    buf = [torch.zeros(size, dtype=dt, device="cuda") for _ in range(3 if post else 2)]
     view = lambda b: torch.as_strided(b, (27, nb, 512), (kst, block_stride, 1), off)  # noqa: E731
     view(buf[0]).copy_(torch.tensor(f0).to(dt))
     vel = [torch.zeros(3 * nb * 512 + off, dtype=mt, device="cuda") for _ in range(2)]
@@ -48,6 +49,7 @@ def run(case, storage, steps, off=0, block_stride=512, pad=0, post=False):
     force = torch.zeros(3, dtype=torch.float64, device="cuda")
     p = capi.StepParams.from_buffer_copy(case.params)
     p.store_post_collision = int(post)
+    p.svv_x_epsilon, p.svv_yz_epsilon = svv
     at = lambda t: t.data_ptr() + off * t.element_size()  # noqa: E731
     for _ in range(steps):
         fl = capi.LevelFields(at(buf[0]), at(buf[1]), at(buf[2]) if post else None, at(rho), at(vel[1]), at(vel[0]),
@@ -167,3 +169,28 @@ def test_face_values_of_extents_inside_a_block(oal, storage, shape):
         assert np.max(np.abs(a - b)) < TOL[storage] * np.max(np.abs(b))
     L.close()
     g.close()
+
+
+WIDE = 2 * (2 ** 31 // 26 + 1)  # elements apart: 27 directions, or 27 blocks, span more than 2^32 elements
+
+
+@pytest.mark.parametrize("svv", [(0.0, 0.0), (0.0, 0.004), (0.003, 0.004)])
+@pytest.mark.parametrize("options", [dict(), dict(omega3=1.1, limiter_type=capi.OAL_LIMITER_POSITIVITY)],
+                         ids=["default", "general_rates"])
+@pytest.mark.parametrize("strides", [dict(dir_stride=WIDE), dict(block_stride=WIDE, dir_stride=512)],
+                         ids=["directions", "blocks"])
+@pytest.mark.parametrize("storage", ["f32", "f64", "f16", "bf16"])
+def test_arrays_past_2_32_elements_keep_their_bits(oal, storage, strides, options, svv):
+    """Spans of more than 2^32 elements take the kernels' 64-bit index instances: the same arithmetic, so the
+    bits of the compact arrays."""
+    import torch
+    case = taylor_green_case(24, c_wale=0.2)
+    for k, v in options.items():
+        setattr(case.params, k, v)
+    try:
+        want = run(case, storage, 2, svv=svv)
+        got = run(case, storage, 2, svv=svv, **strides)
+    finally:
+        torch.cuda.empty_cache()
+    for a, b in zip(got, want):
+        assert np.array_equal(a, b)

@@ -326,3 +326,40 @@ def test_g13_poiseuille_tilted_plates(env):
         assert e[2] < e[1] < e[0], (angle, e)
         assert abs(res[-1][1]) < 0.05, (angle, res[-1])
         assert res[-1][2] < 0.01, (angle, res[-1])
+
+
+class Copies:
+    """`n` copies of a periodic box in one level, each with its own neighbours only."""
+
+    def __init__(self, box, n):
+        self.nocts, self.dx = n * box.nocts, box.dx
+        shift = np.repeat(np.arange(n, dtype=np.int32) * box.nocts, box.nocts * 27)
+        self.onbr = (np.tile(np.asarray(box.onbr, np.int32).reshape(-1), n) + shift).reshape(self.nocts, 27)
+
+
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+def test_level_past_4_gb_keeps_its_bits(env, dt):
+    """A level whose populations pass 4 GB takes the kernels' 64-bit offsets: every copy of a box in it steps
+    to the bits of the box alone (32-bit offsets)."""
+    _, _, octree, _ = env
+    n = (64, 48, 40)
+    box = octree.PeriodicBox(*n)
+    copies = 2 ** 32 // (box.nocts * 8 * 19 * np.dtype(dt).itemsize) + 1
+    cfg = octree.test_case_config(box, precision=dt)
+    p = _params(nu=0.002, sgs=1, sigma=0.98)
+    one = octree.State(box, cfg)
+    one.params = p
+    rho, u, _ = one.initial_fields(shear_layer(n), False)
+    one._upload(rho, u, None)
+    one.advance(3)
+    want = one.state()
+    one.close()
+    many = octree.State(Copies(box, copies), cfg)
+    many.params = p
+    many._upload(np.tile(rho, (copies, 1)), np.tile(u, (copies, 1, 1)), None)
+    many.advance(3)
+    got = many.state()
+    many.close()
+    for a, b in zip(got, want):
+        a = a.reshape(copies, *b.shape)
+        assert all(same_bits(a[i], b) for i in range(copies))
