@@ -1364,6 +1364,16 @@ oal_status oal_geometry_info(const oal_geometry* g, int64_t out[5]) {
   return OAL_OK;
 }
 
+// Whether the interior blocks of caller-owned arrays take the uniform kernel, a second launch behind the
+// general one: it starts when that one's last wave has drained, which a few blocks do not repay. Channels,
+// all blocks in the general kernel against split, us a step: FP32 100 interior blocks (56 x 56 x 48) 31.0
+// against 34.6, 120 (256 x 32 x 32) 47.9 against 46.5, 125 (56^3) 37.2 against 35.4 (FP16 33.1/36.5, 50.8/48.5,
+// 39.6/37.4); FP64, whose two kernels are closer, 432 (112 x 64 x 64) 104 against 106, 504 (128 x 64 x 64) 117
+// against 114. With every block interior there is one launch either way (16^3 FP32 12.0 against 9.5).
+static bool uniform_blocks_pay(const oal_geometry* g, int32_t storage) {
+  return g->n_fast_in > 0 && (g->n_plain == 0 || g->n_fast_in >= (storage == OAL_STORE_F64 ? 448 : 112));
+}
+
 oal_status oal_stream_collide(const oal_geometry* g, const oal_level_fields* fl, const oal_step_params* p, void* stream) {
   if (!g || !fl) return set_error(OAL_E_INVALID_ARG, "null argument");
   CaseParams cp;
@@ -1393,7 +1403,7 @@ oal_status oal_stream_collide(const oal_geometry* g, const oal_level_fields* fl,
   // start on a pair; f_post_collision is the general kernel's
   const size_t pw = 2 * storage_bytes(fl->storage), pm = 2 * macro_bytes(fl->storage);
   auto on = [](const void* q, size_t bytes) { return (uintptr_t)q % bytes == 0; };
-  a.strided = g->n_fast_in > 0 && !((cp.flags & CF_STORE_POST) && a.f_post) && a.f_bstride % 2 == 0 && a.f_kstride % 2 == 0 &&
+  a.strided = uniform_blocks_pay(g, fl->storage) && !((cp.flags & CF_STORE_POST) && a.f_post) && a.f_bstride % 2 == 0 && a.f_kstride % 2 == 0 &&
               a.v_cstride % 2 == 0 && on(a.f_in, pw) && on(a.f_out, pw) && on(a.rho_out, pm) && on(a.vel_out, pm) &&
               on(a.vel_in, pm);
   OAL_CUDA_TRY(launch_by_storage(fl->storage, g, a, PATH_PLAIN, st));

@@ -73,6 +73,11 @@ def cases():
     c = sphere_channel_case(40, 40, 40, diameter=8.0, centre_x=16.0, re=100.0, omega3=1.1,
                             limiter_type=capi.OAL_LIMITER_POSITIVITY)
     yield "general_rates", c
+    # enough interior blocks for a launch of their own: 504, FP64's 448 among them, and 125 of the 112 elsewhere
+    yield "split", sphere_channel_case(128, 64, 64, diameter=16.0, centre_x=32.0, re=100.0)
+    yield "split_rates", sphere_channel_case(128, 64, 64, diameter=16.0, centre_x=32.0, re=100.0, omega3=1.1,
+                                             limiter_type=capi.OAL_LIMITER_POSITIVITY)
+    yield "split_least", sphere_channel_case(56, 56, 56, diameter=8.0, centre_x=16.0, re=100.0)
 
 
 @pytest.mark.parametrize("storage", ["f32", "f64", "f16", "bf16"])
@@ -88,8 +93,9 @@ def test_uniform_and_general_routes_agree(oal, storage, name, case):
 
 
 @pytest.mark.parametrize("kw", [dict(off=1), dict(pad=1), dict(off=1, pad=3)])
-def test_unpaired_arrays_keep_the_general_route(oal, kw):
-    case = sphere_channel_case(40, 40, 40, diameter=8.0, centre_x=16.0, re=100.0)
+@pytest.mark.parametrize("edge", [40, 64])
+def test_unpaired_arrays_keep_the_general_route(oal, kw, edge):
+    case = sphere_channel_case(edge, edge, edge, diameter=8.0, centre_x=16.0, re=100.0)
     want, got = run(case, "f32", STEPS, post=True), run(case, "f32", STEPS, **kw)
     for a, b in zip(got, want):
         assert np.array_equal(a, b)
@@ -116,9 +122,10 @@ OPTIONS = [dict(), dict(inlet_turbulence=0.05, time_step_seed=3), dict(compressi
 @pytest.mark.parametrize("storage", ["f32", "f64"])
 @pytest.mark.parametrize("options", OPTIONS, ids=lambda o: "-".join(o) or "default")
 @pytest.mark.parametrize("holes", [False, True])
-def test_face_values_match_the_ghost_filled_level(oal, storage, options, holes):
+@pytest.mark.parametrize("shape", [(40, 40, 40), (128, 64, 64)])
+def test_face_values_match_the_ghost_filled_level(oal, storage, options, holes, shape):
     from openaerolab_alpha_01_b200.solver import Level
-    case = sphere_channel_case(40, 40, 40, diameter=8.0, centre_x=16.0, re=100.0, **options)
+    case = sphere_channel_case(*shape, diameter=8.0, centre_x=16.0, re=100.0, **options)
     if holes:
         case = holed(case)
     r = np.random.default_rng(5)
