@@ -827,12 +827,14 @@ __device__ __forceinline__ bool alpha_taylor(const Tables& T, const float* sf, c
 // the pair, so sum fe g(y) is a polynomial in coeff_h whose coefficients are 12 sums over the pairs,
 // gathered once. Mass and momentum of s and h are zero (f_eq has the cell's), which leaves the stress
 // moments of s and the energy-flux moments of h. The differences then come out of small quantities
-// alone, and the 12 evaluations are a quartic each. The first dropped term is fe y^5 / 20: at
-// |y| <= kSeriesRoot, which only the light shells reach (w <= 1/432), that is below 4e-8, a tenth of
-// the rounding of the sums it replaces. So the series decides where |y| stays below kSeriesRoot for
-// |coeff_h| <= kRootReach and the root lies there, and below kSeriesFar over the whole bracket
-// (|coeff_h| <= 7), whose far end only has to have the right sign; elsewhere the sums of logarithms
-// decide.
+// alone, and the 12 evaluations are a quartic each. The first dropped term is fe y^5 / 20 a direction: at
+// |y| = kSeriesRoot 4e-8 for the light shells (w <= 1/432), a tenth of the rounding of the sums it
+// replaces, and up to 1.3e-6 for the heaviest. The gate does not ask which shell carries the deviation;
+// where the heavy ones do, up to the gate, the dropped terms move alpha by at most 2.5e-3 (median 1.3e-5,
+// 4,096 cells against the logarithms in 64 bits), less than the bisection's last interval (3.5e-3). So the
+// series decides where |y| stays below kSeriesRoot for |coeff_h| <= kRootReach and the root lies there,
+// and below kSeriesFar over the whole bracket (|coeff_h| <= 7), whose far end only has to have the right
+// sign; elsewhere the sums of logarithms decide.
 constexpr float kSeriesRoot = 0.2f, kSeriesFar = 0.7f, kRootReach = 2.5f;
 struct AlphaSeries {
   float a20 = 0.0f, a11 = 0.0f, a02 = 0.0f, a30 = 0.0f, a21 = 0.0f, a12 = 0.0f, a03 = 0.0f;
@@ -1086,7 +1088,8 @@ __device__ __forceinline__ void svv_axis(const SvvView a, const Tables& T, const
 // What bounds the fast instances: FP32 issue. They run ~5,500 thread-instructions per cell (two to
 // three Newton passes of ~600 and one or two Cholesky solves of ~650, alpha ~1,200, the rest pull,
 // WALE and update) at 168 registers, three CTAs per SM, issue 51 % active (no_instruction and wait
-// stalls: the body is straight-line code). The body is unrolled over the pairs with the 39
+// stalls: the body is straight-line code), with spills of 136 bytes stored and 184 loaded a thread in the
+// plain instance, 298 and 492 in the EDGES ones. The body is unrolled over the pairs with the 39
 // equilibrium values in registers, guards and blends included; HRR, the other alpha solvers and what
 // follows a NaN read the shared columns. Measured on a 96^3 periodic box, two steps per call: 2,660 us with the
 // Newton pass over the basis table, alpha from sums of logarithms over the columns and a trip to

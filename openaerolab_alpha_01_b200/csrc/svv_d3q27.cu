@@ -229,7 +229,10 @@ __device__ __forceinline__ void svv_pairs_filter(const SvvArgs& a, const S* __re
   // the words of a direction: own input, own output, the eight y and z taps, the two x pairs; those of
   // the next directions are on their way while one is filtered (one direction at a time the warps
   // spent two thirds of their time waiting for its ten reads)
-  constexpr int kAhead = KST == 0 ? 0 : sizeof(S) == 2 ? 2 : 1;  // what the registers hold
+  // two (FP32: one) ahead already spill a little at 96 (128) registers: 52 bytes stored, 60 loaded in the
+  // FP16 y-z instance; three 72 and 80. With a run-time stride none is read ahead (104 and 120 at most,
+  // 64-bit offsets 212 and 356)
+  constexpr int kAhead = KST == 0 ? 0 : sizeof(S) == 2 ? 2 : 1;
   W q[kAhead + 1][12];
   auto fetch = [&](int k, W (&d)[12]) {
     const S* fk = fin + (IDX)k * kst;
